@@ -1,6 +1,7 @@
 // Batched engine: many independent beams tracked by one particle launch
 // and one head launch per turn.
 #include "engine_device.cuh"
+#include "convolve.cuh"
 
 // ============================================================ batched beams
 // Many independent beams (ragged particle counts, own RF programme, slicing
@@ -254,6 +255,12 @@ struct blond_batch {
     double2* d_H = nullptr;
     double* d_scale = nullptr;
     double2* d_tw = nullptr;
+    // short profiles: the induced voltages by direct convolution (convolve.cuh)
+    bool conv = false;
+    bb::ConvPlan cplan = {};
+    double* d_hx = nullptr;      // [B][2S-1] impulse responses
+    double* d_cscale = nullptr;  // [B] voltage per unit of response
+    int* d_cticket = nullptr;    // [B] last-block tickets (0 between launches)
     int* d_hist = nullptr;
     double* d_profile = nullptr;
     double* d_vind = nullptr;
@@ -419,6 +426,24 @@ static int launch_batch_profile(blond_batch* q, bool clear, cudaStream_t s) {
 
 static int launch_batch_head(blond_batch* q, cudaStream_t s) {
     if (!q->has_fft) return launch_batch_profile(q, true, s);
+    if (q->conv) {
+        ConvParams C = {};
+        C.p = q->cplan;
+        C.hx = q->d_hx;
+        C.in_i32 = q->d_hist;
+        C.profile_out = q->d_profile;
+        C.out = q->d_vind;
+        C.beam_scale = q->d_cscale;
+        C.table = q->d_table;
+        C.table_f32 = q->precision == BLOND_PREC_F32P64;
+        C.charge = q->charge;
+        C.beam_inv_w = q->d_lik_inv_w;
+        C.bc = q->d_bc;
+        C.turn = q->d_turn;
+        C.ticket = q->d_cticket;
+        C.batch = q->B;
+        return launch_conv(C, s);
+    }
     SpecParams P = {};
     P.p = q->plan;
     P.mode = SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE;
@@ -528,7 +553,8 @@ int blond_batch_destroy(blond_batch* q) {
                     (void*)q->d_bc0, (void*)q->d_lik_inv_w, (void*)q->d_bw, (void*)q->d_bc,
                     (void*)q->d_H, (void*)q->d_scale, (void*)q->d_tw, (void*)q->d_hist,
                     (void*)q->d_profile, (void*)q->d_vind, q->d_table, (void*)q->d_turn,
-                    (void*)q->d_lsb, (void*)q->d_err, (void*)q->d_next_chunk})
+                    (void*)q->d_lsb, (void*)q->d_err, (void*)q->d_next_chunk, (void*)q->d_hx,
+                    (void*)q->d_cscale, (void*)q->d_cticket})
         free_ptr(p);
     delete q;
     return BLOND_OK;
@@ -626,11 +652,17 @@ int blond_batch_set_impedance(blond_batch* q, int64_t n_fft, const double* Z,
     }
     // With at least one beam per two SMs, one CTA per beam when the whole
     // transform fits in its shared memory: no cluster barriers, and the
-    // beams themselves fill the GPU
-    SpecPlan one;
-    if (q->B * 2 >= device_info().sm_count && make_spec_plan(n_fft, one, 1) &&
-        one.smem <= device_info().max_smem_optin)
-        plan = one;
+    // beams themselves fill the GPU.  With fewer, clusters no larger than
+    // the SMs a beam gets (same factors, same bits): 64 beams of 2048 slices
+    // in 16-CTA clusters ran one after another (head and pass of small
+    // beams 106 -> 22 us a turn).
+    SpecPlan small;
+    int max_c = 1;
+    while (2 * max_c * q->B <= device_info().sm_count && max_c < kMaxCluster) max_c *= 2;
+    if ((q->B * 2 >= device_info().sm_count ? make_spec_plan(n_fft, small, 1)
+                                            : shrink_spec_plan(plan, max_c, small)) &&
+        small.smem <= device_info().max_smem_optin)
+        plan = small;
     BB_CHECK_SIZE(n_fft >= q->S && plan.smem <= device_info().max_smem_optin,
                   "batch_set_impedance: n_fft=%lld unsupported for %d slices",
                   (long long)n_fft, q->S);
@@ -645,6 +677,21 @@ int blond_batch_set_impedance(blond_batch* q, int64_t n_fft, const double* Z,
     if ((rc = make_spec_twiddles(plan, &q->d_tw))) return rc;
     q->plan = plan;
     q->has_fft = true;
+    // short profiles: the direct convolution's impulse responses
+    q->conv = false;
+    free_ptr(q->d_hx);
+    q->d_hx = nullptr;
+    if (make_conv_plan(q->S, n_fft, q->B, q->cplan)) {
+        for (int b = 0; b < q->B; ++b) sc[b] = -scale[b];
+        if ((rc = upload((void**)&q->d_cscale, sc.data(), sizeof(double) * q->B))) return rc;
+        if (!q->d_cticket) {
+            BB_CUDA(cudaMalloc((void**)&q->d_cticket, sizeof(int) * q->B));
+            BB_CUDA(cudaMemset(q->d_cticket, 0, sizeof(int) * q->B));
+        }
+        if ((rc = make_conv_response(q->d_H, n_fft, q->S, q->B, &q->d_hx))) return rc;
+        if ((rc = prepare_conv())) return rc;
+        q->conv = true;
+    }
     q->graph_dirty = true;
     return BLOND_OK;
 }

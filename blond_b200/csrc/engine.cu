@@ -16,6 +16,7 @@
 // The turn index lives in device memory, so a CUDA graph of K turns is
 // captured once and replayed.
 #include "engine_device.cuh"
+#include "convolve.cuh"
 
 using namespace bb;
 
@@ -46,6 +47,11 @@ struct blond_engine {
     SpecPlan plan = {};
     double2* d_H = nullptr;
     double2* d_tw = nullptr;  // twiddle tables of the spectral plan
+    // short profiles: the induced voltage by direct convolution (convolve.cuh)
+    bool conv = false;
+    bb::ConvPlan cplan = {};
+    double* d_hx = nullptr;    // impulse response
+    int* d_cticket = nullptr;  // last-block ticket (0 between launches)
     double iv_scale = 0.0;
     bool has_ind = false;
     double* d_ind = nullptr;
@@ -684,7 +690,45 @@ static int launch_interp_table(blond_engine* e, cudaStream_t s, bool head) {
     return BLOND_OK;
 }
 
+// The head of a short profile (make_conv_plan): one launch also with the
+// beam-phase loop or the interpolated tracker's table.
+static int launch_conv_head(blond_engine* e, cudaStream_t s, bool loop) {
+    ConvParams P = {};
+    P.p = e->cplan;
+    P.hx = e->d_hx;
+    if (e->smooth) {
+        P.in_f64 = e->d_profile;  // the smooth deposit's profile (read only)
+    } else {
+        P.in_i32 = e->d_hist;
+        P.profile_out = e->d_profile;
+    }
+    P.out = e->d_vind;
+    P.out_scale = -e->iv_scale;
+    P.ind_coeff = e->has_ind ? e->d_ind : nullptr;
+    P.ind_dbc = e->dbc;
+    P.table = e->d_table;
+    P.table_f32 = e->precision == BLOND_PREC_F32P64;
+    P.charge = e->charge;
+    P.inv_w = e->lik_inv_w;
+    P.bc = e->d_bc;
+    P.interp = e->interp ? 1 : 0;
+    P.rf_v = e->d_V;
+    P.rf_om = e->d_om;
+    P.rf_ph = e->d_ph;
+    P.acc = e->d_acc;
+    P.n_rf = e->n_rf;
+    P.n_turns = e->n_turns;
+    P.turn = e->d_turn;
+    P.ticket = e->d_cticket;
+    P.pdl = e->pdl ? 1 : 0;
+    // as in launch_spectral_head: no table where the particle pass forms its own
+    if (e->variant == 2 && e->precision != BLOND_PREC_F32P64 && !e->has_fb && !e->interp)
+        P.table = nullptr;
+    return loop ? launch_conv_loop(P, fb_args(e), s) : launch_conv(P, s);
+}
+
 static int launch_spectral_head(blond_engine* e, cudaStream_t s, bool loop) {
+    if (e->conv) return launch_conv_head(e, s, loop);
     if (!(e->has_fft || e->has_ind)) {
         if (!e->interp) return launch_profile(e, true, s);
         return launch_interp_table(e, s, true);
@@ -831,7 +875,7 @@ int blond_engine_destroy(blond_engine* e) {
                     (void*)e->d_fb_state, (void*)e->d_fb_trace, (void*)e->d_fb_partials, (void*)e->d_fb_ticket,
                     (void*)e->d_turn, (void*)e->d_err, (void*)e->own_hist, (void*)e->d_profile,
                     (void*)e->d_vind, e->d_table, (void*)e->d_acc64,
-                    (void*)e->d_smooth_ticket})
+                    (void*)e->d_smooth_ticket, (void*)e->d_hx, (void*)e->d_cticket})
         free_ptr(p);
     delete e;
     return BLOND_OK;
@@ -938,6 +982,19 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
     e->plan = plan;
     e->iv_scale = scale;
     e->has_fft = true;
+    // short profiles: the direct convolution's impulse response
+    e->conv = false;
+    free_ptr(e->d_hx);
+    e->d_hx = nullptr;
+    if (make_conv_plan(e->S, n_fft, 1, e->cplan)) {
+        if (!e->d_cticket) {
+            BB_CUDA(cudaMalloc((void**)&e->d_cticket, sizeof(int)));
+            BB_CUDA(cudaMemset(e->d_cticket, 0, sizeof(int)));
+        }
+        if ((rc = make_conv_response(e->d_H, n_fft, e->S, 1, &e->d_hx))) return rc;
+        if ((rc = prepare_conv())) return rc;
+        e->conv = true;
+    }
     e->graph_dirty = true;
     return BLOND_OK;
 }

@@ -115,9 +115,11 @@ __device__ __forceinline__ void fb_add(const FbBins& b, int i, double x, double&
     const bool first = i == 0 || !(b.lo <= b.bc[i - 1]);
     const bool last = i == b.S - 1 || !(b.bc[i + 1] <= b.hi);
     const double w = (first && last) ? 1.0 : ((first || last) ? 0.5 : 1.0);
-    const double base = b.machine != BLOND_FB_SPS_F ? exp(b.alpha * bci) * x : x;
+    // exp(0 * bci) is 1: the unweighted projections leave it out
+    const double base =
+        b.machine != BLOND_FB_SPS_F && b.alpha != 0.0 ? exp(b.alpha * bci) * x : x;
     double sn, cs;
-    sincos(b.omega * bci + b.phi, &sn, &cs);
+    rf_sincos(b.omega * bci + b.phi, &sn, &cs);
     s_sum += w * (base * sn);
     c_sum += w * (base * cs);
 }

@@ -26,6 +26,22 @@ static bool smooth5(int64_t x) {
     return x == 1;
 }
 
+// Shares of a CTA and shared memory for the plan's factors and cluster size:
+// fewest cluster barriers (three buffers) and staged impedance when the
+// shared memory allows, else fall back step by step.
+static void place_spec_plan(SpecPlan& plan) {
+    plan.Bc = plan.M2 / plan.C;
+    plan.Br = plan.M1 / plan.C;
+    const int budget = device_info().max_smem_optin;
+    const int options[4][2] = {{3, 1}, {3, 0}, {2, 1}, {2, 0}};
+    for (const auto& o : options) {
+        plan.nbuf = o[0];
+        plan.prefetch = o[1];
+        plan.smem = spec_layout(plan).total;
+        if (plan.smem <= budget) break;
+    }
+}
+
 bool make_spec_plan(int64_t N, SpecPlan& plan, int max_cluster) {
     if (N < 2 || (N & 1) || N > kMaxClusterFFT) return false;
     const int M = (int)(N / 2);
@@ -54,22 +70,18 @@ bool make_spec_plan(int64_t N, SpecPlan& plan, int max_cluster) {
     plan.M1 = best_m1;
     plan.M2 = M / best_m1;
     plan.C = best_c;
-    plan.Bc = plan.M2 / plan.C;
-    plan.Br = plan.M1 / plan.C;
     radix_schedule(plan.M1, plan.r1, plan.n1);
     radix_schedule(plan.M2, plan.r2, plan.n2);
     plan.L = 1;
     while ((int64_t)plan.L * plan.L < M) plan.L *= 2;
-    // fewest cluster barriers (three buffers) and staged impedance when the
-    // shared memory allows, else fall back step by step
-    const int budget = device_info().max_smem_optin;
-    const int options[4][2] = {{3, 1}, {3, 0}, {2, 1}, {2, 0}};
-    for (const auto& o : options) {
-        plan.nbuf = o[0];
-        plan.prefetch = o[1];
-        plan.smem = spec_layout(plan).total;
-        if (plan.smem <= budget) break;
-    }
+    place_spec_plan(plan);
+    return true;
+}
+
+bool shrink_spec_plan(const SpecPlan& from, int max_cluster, SpecPlan& plan) {
+    plan = from;
+    while (plan.C > max_cluster) plan.C /= 2;
+    place_spec_plan(plan);
     return true;
 }
 
