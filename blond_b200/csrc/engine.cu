@@ -787,6 +787,75 @@ static int launch_turn(blond_engine* e, cudaStream_t s) {
     return e->smooth ? launch_smooth_deposit(e, s) : BLOND_OK;
 }
 
+// Turns whose particles nothing couples (no induced voltage, interpolated
+// kick, loop or smooth slicing) run several to a launch.
+static bool multi_turn(const blond_engine* e) {
+    return !(e->has_fft || e->has_ind || e->interp || e->has_fb || e->smooth);
+}
+
+template <int PREC, int SOLVER>
+static int launch_multi_t(blond_engine* e, const ParticleArgs& a, int first, int turns,
+                          bool deposit, cudaStream_t s) {
+    auto k = e->n_rf == 1   ? particle_kernel_multi<PREC, SOLVER, 1>
+             : e->n_rf == 2 ? particle_kernel_multi<PREC, SOLVER, 2>
+                            : particle_kernel_multi<PREC, SOLVER, 0>;
+    int rc;
+    if ((rc = allow_smem_once(k))) return rc;
+    const size_t smem = sizeof(TurnConsts) * turns +
+                        (deposit && !a.global_hist ? sizeof(int) * (size_t)a.S : 0);
+    // the same number of rounds for every warp: 5e5 pairs are 3.3 rounds of
+    // 1024 threads on 148 SMs, but 4 of 864
+    const int grid = particle_grid(a.n / 2 + 1, kEngineThreads, 1);
+    const int64_t per_sm = (a.n / 2 + grid - 1) / grid;
+    const int64_t rounds = std::max<int64_t>(1, (per_sm + kEngineThreads - 1) / kEngineThreads);
+    const int threads = (int)std::max<int64_t>(32, ((per_sm + rounds - 1) / rounds + 31) / 32 * 32);
+    k<<<grid, threads, smem, s>>>(a, first, turns, deposit ? 1 : 0);
+    BB_LAUNCH_CHECK();
+    return BLOND_OK;
+}
+
+template <int PREC>
+static int launch_multi_p(blond_engine* e, const ParticleArgs& a, int first, int turns,
+                          bool deposit, cudaStream_t s) {
+    switch (e->solver) {
+        case 0: return launch_multi_t<PREC, 0>(e, a, first, turns, deposit, s);
+        case 1: return launch_multi_t<PREC, 1>(e, a, first, turns, deposit, s);
+        default: return launch_multi_t<PREC, 2>(e, a, first, turns, deposit, s);
+    }
+}
+
+// n_turns turns in launches of at most kMultiTurns, evenly split; the
+// histogram, profile and turn counter end as after n_turns single turns.
+static int run_multi(blond_engine* e, int64_t n_turns, cudaStream_t s) {
+    ParticleArgs a = particle_args(e);
+    // the constants of a launch's turns lie before the block's histogram
+    a.global_hist = (size_t)e->S * sizeof(int) + sizeof(TurnConsts) * kMultiTurns + 1024 >
+                    (size_t)device_info().max_smem_optin;
+    BB_CUDA(cudaMemsetAsync(e->d_hist, 0, sizeof(int) * e->S, s));
+    const int64_t launches = (n_turns + kMultiTurns - 1) / kMultiTurns;
+    for (int64_t l = 0; l < launches; ++l) {
+        const int64_t lo = n_turns * l / launches, hi = n_turns * (l + 1) / launches;
+        const bool deposit = l == launches - 1;
+        int rc;
+        switch (e->precision) {
+            case BLOND_PREC_F64:
+                rc = launch_multi_p<PREC_F64>(e, a, (int)lo, (int)(hi - lo), deposit, s);
+                break;
+            case BLOND_PREC_F32P64:
+                rc = launch_multi_p<PREC_F32P64>(e, a, (int)lo, (int)(hi - lo), deposit, s);
+                break;
+            default:
+                rc = launch_multi_p<PREC_Q32P64>(e, a, (int)lo, (int)(hi - lo), deposit, s);
+        }
+        if (rc) return rc;
+    }
+    const int threads = 256;
+    profile_kernel<<<std::min(64, (e->S + threads - 1) / threads), threads, 0, s>>>(
+        e->d_hist, e->d_profile, e->S, 0, e->d_turn, (int)n_turns);
+    BB_LAUNCH_CHECK();
+    return BLOND_OK;
+}
+
 static int check_ready(blond_engine* e) {
     if (!e->rf_set || !e->drift_set || !e->slicing_set || !e->dt) {
         set_error("engine: set_rf, set_drift, set_slicing and bind_beam must all be "
@@ -1519,7 +1588,7 @@ int blond_engine_prepare(blond_engine* e, void* stream) {
     BB_CHECK_ARG(e, "engine_prepare: null engine");
     int rc = check_ready(e);
     if (rc) return rc;
-    if (e->turns_per_graph <= 1) return BLOND_OK;
+    if (e->turns_per_graph <= 1 || multi_turn(e)) return BLOND_OK;
     return ensure_graph(e, as_stream(stream));
 }
 
@@ -1533,6 +1602,11 @@ int blond_engine_run(blond_engine* e, int64_t n_turns, void* stream) {
                   (long long)e->n_turns);
     if (n_turns == 0) return BLOND_OK;
     cudaStream_t s = as_stream(stream);
+    if (n_turns > 1 && multi_turn(e)) {
+        if ((rc = run_multi(e, n_turns, s))) return rc;
+        e->host_turn += n_turns;
+        return BLOND_OK;
+    }
     const int K = e->turns_per_graph;
     int64_t done = 0;
     if (n_turns >= K && K > 1) {

@@ -678,6 +678,89 @@ particle_kernel(const ParticleArgs a) {
     if (!a.global_hist) cluster_flush(sh, a.hist, a.S);
 }
 
+// --------------------------------------------------- several turns per pass
+// Turns without induced voltage, loop or smooth slicing: nothing couples the
+// particles, so each pair stays in registers for n_sub turns and the beam
+// crosses memory once per launch instead of once per turn.  The profile array
+// only ever shows the last turn, so only that turn (deposit = 1) is sliced.
+// Each turn runs track_pair with its own constants, the same operations as
+// one pass per turn.  Bound: FP64 issue (24 float64 operations per particle
+// and turn at one RF system: 133 us for 100 turns of 1e6 particles; measured
+// 180 us, 873 us with two launches per turn).  The turn counter is read, not
+// advanced: `first` is this launch's offset from it.
+// NRF: 1 or 2 RF systems written out, 0 the run-time count.
+constexpr int kMultiTurns = 64;  // turns per launch, at most
+
+template <int PREC, int SOLVER, int NRF>
+__global__ void __launch_bounds__(kEngineThreads, 1)
+particle_kernel_multi(const ParticleArgs a, int first, int n_sub, int deposit_last) {
+    using E = typename Coord<PREC>::E;
+    using E2 = typename Vec2<E>::type;
+    extern __shared__ __align__(16) unsigned char msm[];
+    TurnConsts* const c = reinterpret_cast<TurnConsts*>(msm);
+    int* const sh = reinterpret_cast<int*>(msm + sizeof(TurnConsts) * n_sub);
+    const bool privatise = deposit_last && !a.global_hist;
+    int* const hd = privatise ? sh : a.hist;
+    const long long t0 = *a.turn + first;
+    for (int q = threadIdx.x; q < n_sub; q += blockDim.x) {
+        long long t = t0 + q;
+        t = t < 0 ? 0 : (t >= a.n_turns ? a.n_turns - 1 : t);
+        for (int j = 0; j < a.n_rf; ++j) {
+            c[q].V[j] = a.V[t * a.n_rf + j];
+            c[q].Vf[j] = (float)c[q].V[j];
+            c[q].op[j] = make_double2(a.om[t * a.n_rf + j], a.ph[t * a.n_rf + j]);
+        }
+        c[q].acc = a.acc[t];
+        c[q].d = a.drift[t + 1];
+    }
+    if (privatise)
+        for (int k = threadIdx.x; k < a.S; k += blockDim.x) sh[k] = 0;
+    __syncthreads();
+    ParticleArgs p = {};
+    p.n_rf = NRF ? NRF : a.n_rf;
+    p.charge = a.charge;
+    p.S = a.S;
+    p.lsb = a.lsb;
+    p.inv_lsb = a.inv_lsb;
+    p.err = a.err;
+    double* const dt = reinterpret_cast<double*>(a.dt);
+    E* const dE = reinterpret_cast<E*>(a.dE);
+    const int64_t npairs = a.n / 2;
+    const uint64_t pol = evict_first_policy();
+    auto slice = [&](double t) {
+        const int b = engine_bin(t, a.cut_left, a.inv_w, a.S);
+        if (b >= 0) atomicAdd(&hd[b], 1);
+    };
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npairs;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        double2 tt = stream_load(reinterpret_cast<const double2*>(dt) + i, pol);
+        E2 ee = stream_load(reinterpret_cast<const E2*>(dE) + i, pol);
+        for (int q = 0; q < n_sub; ++q)
+            track_pair<PREC, SOLVER, false, TAB_GLOBAL, NRF == 2>(tt.x, tt.y, ee.x, ee.y, c[q], p,
+                                                                  a.order);
+        stream_store(reinterpret_cast<double2*>(dt) + i, tt, pol);
+        stream_store(reinterpret_cast<E2*>(dE) + i, ee, pol);
+        if (deposit_last) {
+            slice(tt.x);
+            slice(tt.y);
+        }
+    }
+    // odd tail particle
+    if ((a.n & 1) && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        double t = dt[a.n - 1], t2 = t;
+        E e = dE[a.n - 1], e2 = e;
+        for (int q = 0; q < n_sub; ++q)
+            track_pair<PREC, SOLVER, false, TAB_GLOBAL, NRF == 2>(t, t2, e, e2, c[q], p, a.order);
+        dt[a.n - 1] = t;
+        dE[a.n - 1] = e;
+        if (deposit_last) slice(t);
+    }
+    if (!privatise) return;
+    __syncthreads();
+    for (int k = threadIdx.x; k < a.S; k += blockDim.x)
+        if (sh[k]) atomicAdd(&a.hist[k], sh[k]);
+}
+
 // ------------------------------------------------- shared-table plain pass
 // The plain pass with the induced kick's table in shared memory.  F64 and
 // Q32P64 keep only the induced voltage (8 B per slice: 128 KB at 2^14
@@ -1037,16 +1120,16 @@ particle_kernel_tma(const ParticleArgs a, int* err) {
     }
 }
 
-// Profile <- histogram.  With clear, the histogram is zeroed and the turn
-// counter advanced (the head of a turn without induced voltage).
+// Profile <- histogram.  With clear, the histogram is zeroed (the head of a
+// turn without induced voltage); the turn counter, if given, is advanced.
 static __global__ void profile_kernel(int* hist, double* profile, int S, int clear,
-                               long long* turn) {
+                               long long* turn, int turns = 1) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S;
          k += gridDim.x * blockDim.x) {
         profile[k] = (double)hist[k];
         if (clear) hist[k] = 0;
     }
-    if (clear && turn && blockIdx.x == 0 && threadIdx.x == 0) *turn += 1;
+    if (turn && blockIdx.x == 0 && threadIdx.x == 0) *turn += turns;
 }
 
 }  // namespace bb
