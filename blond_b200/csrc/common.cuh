@@ -96,6 +96,39 @@ template <> struct Vec2<double> { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
 template <> struct Vec2<int> { using type = int2; };
 
+// Constants of the sines below.  As double literals each cost two moves per
+// use in the particle passes' loops (they do not fit in registers there);
+// from the constant bank they are operands of the multiply-adds themselves
+// (20 of 150 instructions per particle; 2^16-slice double-RF FP64 pass 181 ->
+// 163 us at 2e7 particles, 1e7-particle pass 61.4 -> 60.2 us).
+static __constant__ double kSin[14] = {
+    6755399441055744.0,       // 1.5 * 2^52
+    0.3183098861837907,       // 1 / pi
+    3.1415926553308964,       // pi = P1 + P2 + P3
+    -1.7411031384001463e-09,
+    -7.00686879617986e-19,
+    2.7314447669863995e-15,   // sin r = r + r^3 P(r^2): P from its highest term
+    -7.643970296798572e-13,
+    1.6058977312464087e-10,
+    -2.5052107616996182e-08,
+    2.7557319219163234e-06,
+    -0.00019841269841254974,
+    0.008333333333333316,
+    -0.16666666666666666,
+    3.141592653589793,        // pi
+};
+static __constant__ double kCos[9] = {
+    -1.5169166967261124e-16,  // cos r = 1 + r^2 Q(r^2): Q from its highest term
+    4.777404889695354e-14,
+    -1.147069401087498e-11,
+    2.0876756238770223e-09,
+    -2.7557319217593045e-07,
+    2.4801587301556646e-05,
+    -0.0013888888888888816,
+    0.041666666666666664,
+    -0.5,
+};
+
 // sin(x) of an RF phase argument.  The FP64 particle passes spend much of
 // their issue slots on this sine, so it is written for the arguments they
 // see (|x| up to ~1e3 rad): Cody-Waite reduction by pi (W. J. Cody and
@@ -116,24 +149,24 @@ __device__ __forceinline__ double rf_sin(double x) {
     // (rounded) quotient to the nearest integer, ties to even, exactly as
     // rint does for |x / pi| < 2^51, and leaves k's parity in the low bit
     // of the shifted sum
-    const double shifter = 6755399441055744.0;  // 1.5 * 2^52
-    const double y = __dmul_rn(x, 0.3183098861837907);  // 1 / pi
+    const double shifter = kSin[0];  // 1.5 * 2^52
+    const double y = __dmul_rn(x, kSin[1]);  // 1 / pi
     const double ks = __dadd_rn(y, shifter);
     const double k = __dsub_rn(ks, shifter);
-    double r = fma(-k, 3.1415926553308964, x);       // P1
-    r = fma(-k, -1.7411031384001463e-09, r);          // P2
-    r = fma(-k, -7.00686879617986e-19, r);            // P3
+    double r = fma(-k, kSin[2], x);       // P1
+    r = fma(-k, kSin[3], r);          // P2
+    r = fma(-k, kSin[4], r);            // P3
     const double r2 = r * r;
     // sin r = r + r^3 P(r^2), P the degree-7 Chebyshev approximation on
     // [0, (pi/2)^2] (gen_sin_coeffs.py; error below 1.3e-18)
-    double p = 2.7314447669863995e-15;
-    p = fma(p, r2, -7.643970296798572e-13);
-    p = fma(p, r2, 1.6058977312464087e-10);
-    p = fma(p, r2, -2.5052107616996182e-08);
-    p = fma(p, r2, 2.7557319219163234e-06);
-    p = fma(p, r2, -0.00019841269841254974);
-    p = fma(p, r2, 0.008333333333333316);
-    p = fma(p, r2, -0.16666666666666666);
+    double p = kSin[5];
+    p = fma(p, r2, kSin[6]);
+    p = fma(p, r2, kSin[7]);
+    p = fma(p, r2, kSin[8]);
+    p = fma(p, r2, kSin[9]);
+    p = fma(p, r2, kSin[10]);
+    p = fma(p, r2, kSin[11]);
+    p = fma(p, r2, kSin[12]);
     double s = fma(r * r2, p, r);
     return (__double2loint(ks) & 1) ? -s : s;
 }
@@ -143,32 +176,32 @@ __device__ __forceinline__ double rf_sin(double x) {
 // [0, (pi/2)^2] (gen_sin_coeffs.py; within 1.6e-16 absolute).  Same range
 // as rf_sin; no branch.
 __device__ __forceinline__ void rf_sincos(double x, double* sp, double* cp) {
-    const double shifter = 6755399441055744.0;  // 1.5 * 2^52
-    const double y = __dmul_rn(x, 0.3183098861837907);
+    const double shifter = kSin[0];  // 1.5 * 2^52
+    const double y = __dmul_rn(x, kSin[1]);
     const double ks = __dadd_rn(y, shifter);
     const double k = __dsub_rn(ks, shifter);
-    double r = fma(-k, 3.1415926553308964, x);
-    r = fma(-k, -1.7411031384001463e-09, r);
-    r = fma(-k, -7.00686879617986e-19, r);
+    double r = fma(-k, kSin[2], x);
+    r = fma(-k, kSin[3], r);
+    r = fma(-k, kSin[4], r);
     const double r2 = r * r;
-    double p = 2.7314447669863995e-15;
-    p = fma(p, r2, -7.643970296798572e-13);
-    p = fma(p, r2, 1.6058977312464087e-10);
-    p = fma(p, r2, -2.5052107616996182e-08);
-    p = fma(p, r2, 2.7557319219163234e-06);
-    p = fma(p, r2, -0.00019841269841254974);
-    p = fma(p, r2, 0.008333333333333316);
-    p = fma(p, r2, -0.16666666666666666);
+    double p = kSin[5];
+    p = fma(p, r2, kSin[6]);
+    p = fma(p, r2, kSin[7]);
+    p = fma(p, r2, kSin[8]);
+    p = fma(p, r2, kSin[9]);
+    p = fma(p, r2, kSin[10]);
+    p = fma(p, r2, kSin[11]);
+    p = fma(p, r2, kSin[12]);
     const double s = fma(r * r2, p, r);
-    double q = -1.5169166967261124e-16;
-    q = fma(q, r2, 4.777404889695354e-14);
-    q = fma(q, r2, -1.147069401087498e-11);
-    q = fma(q, r2, 2.0876756238770223e-09);
-    q = fma(q, r2, -2.7557319217593045e-07);
-    q = fma(q, r2, 2.4801587301556646e-05);
-    q = fma(q, r2, -0.0013888888888888816);
-    q = fma(q, r2, 0.041666666666666664);
-    q = fma(q, r2, -0.5);
+    double q = kCos[0];
+    q = fma(q, r2, kCos[1]);
+    q = fma(q, r2, kCos[2]);
+    q = fma(q, r2, kCos[3]);
+    q = fma(q, r2, kCos[4]);
+    q = fma(q, r2, kCos[5]);
+    q = fma(q, r2, kCos[6]);
+    q = fma(q, r2, kCos[7]);
+    q = fma(q, r2, kCos[8]);
     const double c = fma(r2, q, 1.0);
     const bool odd = (__double2loint(ks) & 1) != 0;
     *sp = odd ? -s : s;
@@ -181,10 +214,10 @@ __device__ __forceinline__ void rf_sincos(double x, double* sp, double* cp) {
 // float, P the degree-4 Chebyshev approximation on [0, (pi/2)^2]
 // (gen_sin_coeffs.py; within 2 float ulps).  No branch.
 __device__ __forceinline__ float rf_sinf(double x) {
-    const double shifter = 6755399441055744.0;  // 1.5 * 2^52
-    const double ks = __dadd_rn(__dmul_rn(x, 0.3183098861837907), shifter);
+    const double shifter = kSin[0];  // 1.5 * 2^52
+    const double ks = __dadd_rn(__dmul_rn(x, kSin[1]), shifter);
     const double k = __dsub_rn(ks, shifter);
-    const float r = (float)fma(-k, 3.141592653589793, x);
+    const float r = (float)fma(-k, kSin[13], x);
     const float r2 = r * r;
     float p = -2.408019028621311e-08f;
     p = fmaf(p, r2, 2.75364641311171e-06f);
