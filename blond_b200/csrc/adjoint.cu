@@ -46,10 +46,12 @@
 #include "../../include/blond_b200.h"
 #include "common.cuh"
 #include "spectral.cuh"
+#include "convolve.cuh"
 
 namespace bb {
 
-constexpr int kAdjThreads = 256;
+constexpr int kAdjThreads = 512;
+constexpr int kAdjBlocks = 2;  // per SM
 constexpr int kAdjMaxRf = 4;
 
 struct AdjTurn {
@@ -105,16 +107,47 @@ __device__ __forceinline__ void cic_deposit(u64* h, int S, double t, double bc0,
     if (j + 1 < S && w1) atomicAdd(&h[j + 1], w1);
 }
 
-__device__ __forceinline__ void zero_shared(u64* h, int S) {
-    for (int k = threadIdx.x; k < S; k += blockDim.x) h[k] = 0ull;
+// The same deposit into a block's shared memory.  A 64-bit shared atomic is a
+// compare-and-swap loop (forward turn of 2e6 particles 22 us with it, 11 us
+// without a deposit), so the block keeps, per cell j (particles with floor(f)
+// = j, slot j + 1), the count and the sum of w1 in two 32-bit words with the
+// carry passed on: three native atomics.  flush_split forms the bins,
+// sum w0 = count 2^b - sum w1, exactly as the 64-bit sums would.
+struct SplitHist {
+    unsigned *cnt, *lo, *hi;  // S + 1 slots each
+};
+__device__ __forceinline__ SplitHist split_hist(void* sh, int S) {
+    unsigned* p = static_cast<unsigned*>(sh);
+    return {p, p + (S + 1), p + 2 * (S + 1)};
 }
-__device__ __forceinline__ void flush_shared(const u64* h, u64* g, int S) {
-    for (int k = threadIdx.x; k < S; k += blockDim.x)
-        if (h[k]) atomicAdd(&g[k], h[k]);
+__host__ __device__ inline size_t split_bytes(int S) {
+    return (12 * (size_t)(S + 1) + 15) & ~(size_t)15;
 }
-__device__ __forceinline__ void zero_shared(double* h, int S) {
-    for (int k = threadIdx.x; k < S; k += blockDim.x) h[k] = 0.0;
+__device__ __forceinline__ void zero_split(const SplitHist& h, int S) {
+    for (int k = threadIdx.x; k < 3 * (S + 1); k += blockDim.x) h.cnt[k] = 0u;
 }
+__device__ __forceinline__ void split_deposit(const SplitHist& h, int S, double t, double bc0,
+                                              double inv_w, double scale) {
+    const double f = (t - bc0) * inv_w;
+    if (!(f > -1.0 && f < (double)S)) return;  // also drops NaN
+    const int j = __double2int_rd(f);
+    const u64 w1 = (u64)__double2ll_rn((f - (double)j) * scale);
+    const unsigned lo = (unsigned)w1;
+    unsigned hi = (unsigned)(w1 >> 32);
+    atomicAdd(&h.cnt[j + 1], 1u);
+    const unsigned old = atomicAdd(&h.lo[j + 1], lo);
+    if (old + lo < old) ++hi;
+    if (hi) atomicAdd(&h.hi[j + 1], hi);
+}
+__device__ __forceinline__ void flush_split(const SplitHist& h, u64* g, int S, int bits) {
+    for (int k = threadIdx.x; k < S; k += blockDim.x) {
+        const u64 here = ((u64)h.hi[k + 1] << 32) + h.lo[k + 1];
+        const u64 below = ((u64)h.hi[k] << 32) + h.lo[k];
+        const u64 v = ((u64)h.cnt[k + 1] << bits) - here + below;
+        if (v) atomicAdd(&g[k], v);
+    }
+}
+
 __device__ __forceinline__ void flush_shared(const double* h, double* g, int S) {
     for (int k = threadIdx.x; k < S; k += blockDim.x)
         if (h[k] != 0.0) atomicAdd(&g[k], h[k]);
@@ -127,19 +160,26 @@ __global__ void fixed_to_counts_kernel(double* p, int S, int bits) {
         p[k] = ldexp((double)reinterpret_cast<const u64*>(p)[k], -bits);
 }
 
+__global__ void fixed_to_counts_from_kernel(const u64* raw, double* p, int S, int bits) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x)
+        p[k] = ldexp((double)raw[k], -bits);
+}
+
 __global__ void __launch_bounds__(kAdjThreads)
 adj_deposit_kernel(const double* __restrict__ dt, int64_t n, int S, double bc0, double inv_w,
                    int smem_hist, int bits, u64* __restrict__ prof) {
-    extern __shared__ u64 shq[];
-    u64* sh = shq;
-    u64* h = smem_hist ? sh : prof;
-    if (smem_hist) zero_shared(sh, S);
+    extern __shared__ __align__(16) unsigned char shq[];
+    const SplitHist h = split_hist(shq, S);
+    if (smem_hist) zero_split(h, S);
     __syncthreads();
+    const double scale = ldexp(1.0, bits);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        cic_deposit(h, S, dt[i], bc0, inv_w, bits, ldexp(1.0, bits));
+         i += (int64_t)gridDim.x * blockDim.x) {
+        if (smem_hist) split_deposit(h, S, dt[i], bc0, inv_w, scale);
+        else cic_deposit(prof, S, dt[i], bc0, inv_w, bits, scale);
+    }
     __syncthreads();
-    if (smem_hist) flush_shared(sh, prof, S);
+    if (smem_hist) flush_split(h, prof, S, bits);
 }
 
 // Converts the fixed-point profile to counts in the block that finishes
@@ -159,12 +199,42 @@ __device__ void convert_when_last(u64* prof, int S, int bits, unsigned* done) {
     if (threadIdx.x == 0) *done = 0u;
 }
 
+// One turn of one particle, as the forward map takes it (vind may be null).
+template <int PREC, int NRF>
+__device__ __forceinline__ void adj_step(double& t, typename AdjE<PREC>::E& e, const AdjTurn& T,
+                                         const double* vind, const double* sV, const double* sOm,
+                                         const double* sPh, double acc, double drift_c) {
+    using E = typename AdjE<PREC>::E;
+    const double q = T.charge;
+    if (vind) {
+        const double f = (t - T.bc0) * T.inv_w;
+        if (f >= 0.0 && f < (double)(T.S - 1)) {
+            const int k = __double2int_rd(f);
+            const double w = f - (double)k;
+            e += (E)(q * (vind[k] * (1.0 - w) + vind[k + 1] * w));
+        }
+    }
+    if (PREC == BLOND_PREC_F64) {
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < NRF; ++j) s += sV[j] * sin(fma(sOm[j], t, sPh[j]));
+        e += (E)(q * s + acc);
+    } else {
+        // the engine's F32P64 sine: reduction in double, polynomial in float
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NRF; ++j) s += (float)sV[j] * rf_sinf(fma(sOm[j], t, sPh[j]));
+        e += (E)q * s + (E)acc;
+    }
+    t = t + drift_c * (double)e;
+}
+
 // NRF: the number of RF harmonics, a template parameter so that every
 // harmonic's arithmetic is issued only when it exists (a runtime count
 // under an unrolled loop to kAdjMaxRf left the unused harmonics' sines
 // issued under predicates).
 template <int PREC, int NRF>
-__global__ void __launch_bounds__(kAdjThreads)
+__global__ void __launch_bounds__(kAdjThreads, kAdjBlocks)
 adj_forward_kernel(const AdjTurn T, const double* dt_in, const void* dE_in, double* dt_out,
                    void* dE_out, u64* prof_out, unsigned* done) {
     using E = typename AdjE<PREC>::E;
@@ -172,7 +242,7 @@ adj_forward_kernel(const AdjTurn T, const double* dt_in, const void* dE_in, doub
     // next grid may launch now; the programme and shared memory are set up
     // before this grid waits for the one before it
     pdl_launch_dependents();
-    extern __shared__ u64 shf[];
+    extern __shared__ __align__(16) unsigned char shf[];
     __shared__ double sV[kAdjMaxRf], sOm[kAdjMaxRf], sPh[kAdjMaxRf];
     if (threadIdx.x < T.n_rf) {
         sV[threadIdx.x] = T.V[threadIdx.x];
@@ -181,53 +251,150 @@ adj_forward_kernel(const AdjTurn T, const double* dt_in, const void* dE_in, doub
     }
     const bool dep = prof_out != nullptr;
     const bool hsm = dep && T.smem_hist;
-    u64* h = hsm ? shf : prof_out;
-    if (hsm) zero_shared(shf, T.S);
+    const SplitHist h = split_hist(shf, T.S);
+    if (hsm) zero_split(h, T.S);
     pdl_wait();  // coordinates, induced voltage and counter of the grids before
     const double* vind = T.vind;
     if (vind && T.vind_smem) {
-        double* sv = reinterpret_cast<double*>(shf + (hsm ? T.S : 0));
+        double* sv = reinterpret_cast<double*>(shf + (hsm ? split_bytes(T.S) : 0));
         for (int k = threadIdx.x; k < T.S; k += blockDim.x) sv[k] = T.vind[k];
         vind = sv;
     }
     __syncthreads();
     const E* dEi = static_cast<const E*>(dE_in);
     E* dEo = static_cast<E*>(dE_out);
-    const double q = T.charge;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < T.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        double t = dt_in[i];
-        E e = dEi[i];
-        if (vind) {
-            const double f = (t - T.bc0) * T.inv_w;
-            if (f >= 0.0 && f < (double)(T.S - 1)) {
-                const int k = __double2int_rd(f);
-                const double w = f - (double)k;
-                e += (E)(q * (vind[k] * (1.0 - w) + vind[k + 1] * w));
-            }
+    // the next two particles are on their way while one is computed
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double t1 = i < T.n ? dt_in[i] : 0.0, t2 = i + stride < T.n ? dt_in[i + stride] : 0.0;
+    E e1 = i < T.n ? dEi[i] : E(0), e2 = i + stride < T.n ? dEi[i + stride] : E(0);
+    for (; i < T.n; i += stride) {
+        double t = t1;
+        E e = e1;
+        t1 = t2;
+        e1 = e2;
+        if (i + 2 * stride < T.n) {
+            t2 = dt_in[i + 2 * stride];
+            e2 = dEi[i + 2 * stride];
         }
-        if (PREC == BLOND_PREC_F64) {
-            double s = 0.0;
-#pragma unroll
-            for (int j = 0; j < NRF; ++j) s += sV[j] * sin(fma(sOm[j], t, sPh[j]));
-            e += (E)(q * s + T.acc);
-        } else {
-            // the engine's F32P64 sine: reduction in double, polynomial in float
-            float s = 0.0f;
-#pragma unroll
-            for (int j = 0; j < NRF; ++j) s += (float)sV[j] * rf_sinf(fma(sOm[j], t, sPh[j]));
-            e += (E)q * s + (E)T.acc;
-        }
-        t = t + T.drift_c * (double)e;
+        adj_step<PREC, NRF>(t, e, T, vind, sV, sOm, sPh, T.acc, T.drift_c);
         dt_out[i] = t;
         dEo[i] = e;
-        if (dep) cic_deposit(h, T.S, t, T.bc0, T.inv_w, T.fix_bits, T.fix_scale);
+        if (hsm) split_deposit(h, T.S, t, T.bc0, T.inv_w, T.fix_scale);
+        else if (dep) cic_deposit(prof_out, T.S, t, T.bc0, T.inv_w, T.fix_bits, T.fix_scale);
     }
     if (hsm) {
         __syncthreads();
-        flush_shared(shf, prof_out, T.S);
+        flush_split(h, prof_out, T.S, T.fix_bits);
     }
     if (dep && done) convert_when_last(prof_out, T.S, T.fix_bits, done);
+}
+
+// The turn-start coordinates of up to kAdjSegTurns turns of a segment: with
+// their induced voltages stored, nothing couples the particles, so R of a
+// thread stay in registers for all the turns and only dt is written each turn
+// (states[q] at the start of turn q, states[n_sub] at the end).  Bound: those
+// writes, 8 B per particle and turn (2e6 particles: 2.5 us a turn; one pass
+// per turn took 11).  Each turn's voltages come to shared memory two turns
+// ahead (three buffers, one barrier a turn).  The same operations as
+// adj_forward_kernel, so the same bits.
+constexpr int kAdjSegTurns = 64;
+constexpr int kAdjSegThreads = 512;
+
+struct AdjSegment {
+    AdjTurn T;
+    int n_sub;
+    const double* vind;  // [n_sub][S] or nullptr
+    int smem_vind;
+    double acc[kAdjSegTurns], drift_c[kAdjSegTurns];
+};
+
+__device__ __forceinline__ void adj_copy8(double* smem, const double* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+
+template <int PREC, int NRF, int R>
+__global__ void __launch_bounds__(kAdjSegThreads, 2)
+adj_segment_kernel(const AdjSegment G, const double* dt_in, const void* dE_in, double* states,
+                   void* dE_out) {
+    using E = typename AdjE<PREC>::E;
+    extern __shared__ double shv[];
+    __shared__ double sV[kAdjSegTurns][kAdjMaxRf], sOm[kAdjSegTurns][kAdjMaxRf],
+        sPh[kAdjSegTurns][kAdjMaxRf];
+    const AdjTurn& T = G.T;
+    const int S = T.S;
+    for (int x = threadIdx.x; x < G.n_sub * T.n_rf; x += blockDim.x) {
+        const int q = x / T.n_rf, j = x - q * T.n_rf;
+        sV[q][j] = T.V[x];
+        sOm[q][j] = T.om[x];
+        sPh[q][j] = T.ph[x];
+    }
+    const E* const ein = static_cast<const E*>(dE_in);
+    E* const eout = static_cast<E*>(dE_out);
+    const bool staged = G.vind && G.smem_vind;
+    auto stage = [&](int q) {
+        if (q < G.n_sub)
+            for (int k = threadIdx.x; k < S; k += blockDim.x)
+                adj_copy8(shv + (q % 3) * S + k, G.vind + (size_t)q * S + k);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int64_t tile = (int64_t)gridDim.x * blockDim.x;
+    // every thread of a block runs the same tiles (the barriers need them)
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < T.n; i0 += R * tile) {
+        double t[R];
+        E e[R];
+        const int64_t i = i0 + threadIdx.x;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool in = i + r * tile < T.n;
+            t[r] = in ? dt_in[i + r * tile] : 0.0;
+            e[r] = in ? ein[i + r * tile] : E(0);
+            if (in) states[i + r * tile] = t[r];
+        }
+        __syncthreads();  // the programme, and the last tile's voltages are free
+        if (staged) {
+            stage(0);
+            stage(1);
+        }
+        for (int q = 0; q < G.n_sub; ++q) {
+            const double* v = G.vind ? G.vind + (size_t)q * S : nullptr;
+            if (staged) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                __syncthreads();
+                stage(q + 2);  // into the buffer of turn q - 1
+                v = shv + (q % 3) * S;
+            }
+            double* const out = states + (size_t)(q + 1) * T.n;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                adj_step<PREC, NRF>(t[r], e[r], T, v, sV[q], sOm[q], sPh[q], G.acc[q],
+                                    G.drift_c[q]);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (i + r * tile < T.n) out[i + r * tile] = t[r];
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (i + r * tile < T.n) eout[i + r * tile] = e[r];
+    }
+    if (staged) asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// accum[k] += sum_t P_t[k] conj(L_t[k]) over n_rows rows of M1 values.
+__global__ void adj_accumulate_kernel(const double2* P, const double2* L, int64_t M1, int n_rows,
+                                      double2* accum) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < M1;
+         k += (int64_t)gridDim.x * blockDim.x) {
+        double re = 0.0, im = 0.0;
+        for (int t = n_rows - 1; t >= 0; --t) {
+            const double2 p = P[t * M1 + k], l = L[t * M1 + k];
+            re += p.x * l.x + p.y * l.y;
+            im += p.y * l.x - p.x * l.y;
+        }
+        accum[k].x += re;
+        accum[k].y += im;
+    }
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -237,11 +404,11 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // One backward turn (kick = 1), or only the deposit adjoint of a profile
-// at dt_next (kick = 0).  Shared memory: lambda_p_next copy, then the
-// block's lambda_V accumulator (S doubles each, when smem_hist), then a
-// copy of the turn's induced voltage (when vind_smem).
+// at dt_next (kick = 0).  Bound: latency and the shared FP64 additions
+// (compare-and-swap loops, 10 of 34 us at 2e6 particles); prefetching the next
+// particle and one gather per table took it from 37.5 us (50 cold).
 template <int NRF>
-__global__ void __launch_bounds__(kAdjThreads)
+__global__ void __launch_bounds__(kAdjThreads, kAdjBlocks)
 adj_backward_kernel(const AdjTurn T, int kick, const double* __restrict__ dt,
                     const double* __restrict__ dt_next, const double* __restrict__ lam_p_next,
                     double* __restrict__ lam_dt, double* __restrict__ lam_dE,
@@ -251,47 +418,61 @@ adj_backward_kernel(const AdjTurn T, int kick, const double* __restrict__ dt,
     __shared__ double red[kAdjThreads / 32][2 * kAdjMaxRf];
     const int S = T.S;
     const bool sm = T.smem_hist != 0;
-    double* lp = sm ? sh : const_cast<double*>(lam_p_next);
-    double* lv = sm ? sh + S : lam_v;
-    const double* vind = T.vind;
+    // shared memory: the deposit adjoint's slopes (cell j at j + 1), the
+    // block's lambda_V, then the voltage's steps: one gather each a particle
+    double* const slope = sh;
+    double* lv = sm ? sh + S + 1 : lam_v;
+    double* const step = sh + 2 * S + 1;
+    const double q = T.charge;
+    auto slope_at = [&](int j) {  // of cell j in [-1, S - 1]
+        const double a = j >= 0 ? lam_p_next[j] : 0.0;
+        const double b = j + 1 < S ? lam_p_next[j + 1] : 0.0;
+        return (b - a) * T.inv_w;
+    };
     pdl_launch_dependents();  // as in adj_forward_kernel
     if (kick && threadIdx.x < T.n_rf) {
         sV[threadIdx.x] = T.V[threadIdx.x];
         sOm[threadIdx.x] = T.om[threadIdx.x];
         sPh[threadIdx.x] = T.ph[threadIdx.x];
     }
+    const bool steps = T.vind && T.vind_smem;
+    if (sm)
+        for (int k = threadIdx.x; k < S; k += blockDim.x) lv[k] = 0.0;
+    if (steps)  // the voltages were stored by the forward run
+        for (int k = threadIdx.x; k < S - 1; k += blockDim.x)
+            step[k] = q * (T.vind[k + 1] - T.vind[k]);
     pdl_wait();  // the adjoint and coordinates of the grids before
-    if (sm) {
-        for (int k = threadIdx.x; k < S; k += blockDim.x) {
-            sh[k] = lam_p_next ? lam_p_next[k] : 0.0;
-            sh[S + k] = 0.0;
-        }
-    }
-    if (vind && T.vind_smem) {
-        double* sv = sh + 2 * S;
-        for (int k = threadIdx.x; k < S; k += blockDim.x) sv[k] = T.vind[k];
-        vind = sv;
-    }
+    if (sm && lam_p_next)
+        for (int k = threadIdx.x; k <= S; k += blockDim.x) slope[k] = slope_at(k - 1);
     __syncthreads();
-    const double q = T.charge;
     double gv[kAdjMaxRf], gp[kAdjMaxRf];
 #pragma unroll
     for (int j = 0; j < kAdjMaxRf; ++j) gv[j] = gp[j] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < T.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        double ldt = lam_dt[i];
-        double ldE = lam_dE[i];
+    // the next particle's values are on their way while one is computed
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double n_ldt = 0.0, n_ldE = 0.0, n_t = 0.0, n_tn = 0.0;
+    auto fetch = [&](int64_t x) {
+        if (x < T.n) {
+            n_ldt = lam_dt[x];
+            n_ldE = lam_dE[x];
+            if (kick) n_t = dt[x];
+            if (lam_p_next) n_tn = dt_next[x];
+        }
+    };
+    fetch(i);
+    for (; i < T.n; i += stride) {
+        double ldt = n_ldt, ldE = n_ldE;
+        const double t = n_t, t_next = n_tn;
+        fetch(i + stride);
         if (lam_p_next) {
-            const double f = (dt_next[i] - T.bc0) * T.inv_w;
+            const double f = (t_next - T.bc0) * T.inv_w;
             if (f > -1.0 && f < (double)S) {
                 const int j = __double2int_rd(f);
-                const double a = j >= 0 ? lp[j] : 0.0;
-                const double b = j + 1 < S ? lp[j + 1] : 0.0;
-                ldt += (b - a) * T.inv_w;
+                ldt += sm ? slope[j + 1] : slope_at(j);
             }
         }
         if (kick) {
-            const double t = dt[i];
             const double lE = ldE + T.drift_c * ldt;
             double dg = 0.0;
 #pragma unroll
@@ -305,12 +486,12 @@ adj_backward_kernel(const AdjTurn T, int kick, const double* __restrict__ dt,
                 gp[j] += lE * sV[j] * c;
             }
             dg *= q;
-            if (vind) {
+            if (T.vind) {
                 const double f = (t - T.bc0) * T.inv_w;
                 if (f >= 0.0 && f < (double)(S - 1)) {
                     const int k = __double2int_rd(f);
                     const double w = f - (double)k;
-                    dg += q * (vind[k + 1] - vind[k]) * T.inv_w;
+                    dg += (steps ? step[k] : q * (T.vind[k + 1] - T.vind[k])) * T.inv_w;
                     atomicAdd(&lv[k], lE * q * (1.0 - w));
                     atomicAdd(&lv[k + 1], lE * q * w);
                 }
@@ -346,8 +527,11 @@ adj_backward_kernel(const AdjTurn T, int kick, const double* __restrict__ dt,
 static int adj_smem_limit() { return (device_info().max_smem_optin - 4096) / 16; }
 
 // Shared memory a block may take for its copy of the induced voltage (with
-// the arrays it holds anyway), so that four blocks still fit on an SM.
-constexpr size_t kAdjVindSmem = 48 * 1024;
+// the arrays it holds anyway), so that kAdjBlocks still fit on an SM.
+constexpr size_t kAdjVindSmem = 96 * 1024;
+// Shared memory of adj_segment_kernel's three voltage buffers (two blocks per
+// SM); longer profiles gather from global memory.
+constexpr size_t kAdjSegSmem = 100 * 1024;
 
 template <typename K>
 static int adj_allow_smem(K kernel, bool* done) {
@@ -422,7 +606,7 @@ static auto adj_backward_for(int n_rf) {
 
 // One forward turn.  With a counter (`done`, zero between launches) the
 // last block converts the deposited profile to counts; without one a
-// second launch does.
+// second launch does, unless the caller wants the fixed-point deposit (raw).
 static int adj_forward_launch(int precision, const double* dt_in, const void* dE_in,
                               double* dt_out, void* dE_out, int64_t n, int n_rf,
                               const double* voltage, const double* omega_rf,
@@ -430,7 +614,7 @@ static int adj_forward_launch(int precision, const double* dt_in, const void* dE
                               double drift_coeff, const double* induced_voltage,
                               int n_slices, double bin_center0, double inv_bin_width,
                               double* profile_out, unsigned* done, void* stream,
-                              bool pdl = false) {
+                              bool pdl = false, bool raw = false) {
     BB_CHECK_ARG(precision == BLOND_PREC_F64 || precision == BLOND_PREC_F32P64,
                  "adjoint_forward_turn: unknown precision %d", precision);
     BB_CHECK_SIZE(n_rf >= 0 && n_rf <= kAdjMaxRf, "adjoint_forward_turn: n_rf=%d not in "
@@ -456,10 +640,10 @@ static int adj_forward_launch(int precision, const double* dt_in, const void* dE
     T.smem_hist = n_slices <= adj_smem_limit() ? 1 : 0;
     T.fix_bits = fixed_bits(n);
     T.fix_scale = ldexp(1.0, T.fix_bits);
-    const size_t hist = profile_out && T.smem_hist ? sizeof(u64) * n_slices : 0;
+    const size_t hist = profile_out && T.smem_hist ? split_bytes(n_slices) : 0;
     T.vind_smem = induced_voltage && hist + sizeof(double) * n_slices <= kAdjVindSmem;
     const size_t smem = hist + (T.vind_smem ? sizeof(double) * n_slices : 0);
-    const int grid = particle_grid(n, kAdjThreads, 4);
+    const int grid = particle_grid(n, kAdjThreads, kAdjBlocks);
     cudaStream_t s = as_stream(stream);
     u64* prof = reinterpret_cast<u64*>(profile_out);
     int rc;
@@ -468,7 +652,7 @@ static int adj_forward_launch(int precision, const double* dt_in, const void* dE
     if ((rc = adj_allow_smem(k))) return rc;
     if ((rc = adj_launch(k, grid, smem, s, pdl, T, dt_in, dE_in, dt_out, dE_out, prof, done)))
         return rc;
-    if (profile_out && !done) {
+    if (profile_out && !done && !raw) {
         fixed_to_counts_kernel<<<(n_slices + 255) / 256, 256, 0, s>>>(profile_out, n_slices,
                                                                       T.fix_bits);
         BB_LAUNCH_CHECK();
@@ -512,10 +696,25 @@ static int adj_backward_launch(const double* dt, const double* dt_next, int64_t 
     int rc;
     const auto k = adj_backward_for(kick ? n_rf : 0);
     if ((rc = adj_allow_smem(k))) return rc;
-    const size_t smem = T.smem_hist ? (T.vind_smem ? 3 : 2) * sizeof(double) * n_slices : 0;
-    const int grid = particle_grid(n, kAdjThreads, 4);
+    const size_t smem =
+        T.smem_hist ? sizeof(double) * ((T.vind_smem ? 3 : 2) * (size_t)n_slices + 1) : 0;
+    const int grid = particle_grid(n, kAdjThreads, kAdjBlocks);
     return adj_launch(k, grid, smem, as_stream(stream), pdl, T, kick, dt, dt_next, lam_p_next,
                       lam_dt, lam_dE, lam_v, grad_rf);
+}
+
+// Fixed-point deposit of dt into prof (added to what it holds).
+static int adj_deposit_launch(const double* dt, int64_t n, int n_slices, double bin_center0,
+                              double inv_bin_width, u64* prof, cudaStream_t s) {
+    static bool done[64] = {false};
+    int rc;
+    if ((rc = adj_allow_smem(adj_deposit_kernel, done))) return rc;
+    const int sm = n_slices <= adj_smem_limit() ? 1 : 0;
+    const int grid = particle_grid(n, kAdjThreads, kAdjBlocks);
+    adj_deposit_kernel<<<grid, kAdjThreads, sm ? split_bytes(n_slices) : 0, s>>>(
+        dt, n, n_slices, bin_center0, inv_bin_width, sm, fixed_bits(n), prof);
+    BB_LAUNCH_CHECK();
+    return BLOND_OK;
 }
 
 }  // namespace bb
@@ -529,16 +728,10 @@ int blond_adjoint_deposit(const double* dt, int64_t n, int n_slices, double bin_
     BB_CHECK_ARG(n >= 0 && n_slices >= 1, "adjoint_deposit: bad size");
     BB_CHECK_ARG(profile && (n == 0 || dt), "adjoint_deposit: null pointer");
     if (n == 0) return BLOND_OK;
-    static bool done[64] = {false};
-    int rc;
-    if ((rc = adj_allow_smem(adj_deposit_kernel, done))) return rc;
-    const int sm = n_slices <= adj_smem_limit() ? 1 : 0;
-    const int grid = particle_grid(n, kAdjThreads, 4);
     cudaStream_t s = as_stream(stream);
-    adj_deposit_kernel<<<grid, kAdjThreads, sm ? sizeof(u64) * n_slices : 0, s>>>(
-        dt, n, n_slices, bin_center0, inv_bin_width, sm, fixed_bits(n),
-        reinterpret_cast<u64*>(profile));
-    BB_LAUNCH_CHECK();
+    const int rc = adj_deposit_launch(dt, n, n_slices, bin_center0, inv_bin_width,
+                                      reinterpret_cast<u64*>(profile), s);
+    if (rc) return rc;
     fixed_to_counts_kernel<<<(n_slices + 255) / 256, 256, 0, s>>>(profile, n_slices,
                                                                   fixed_bits(n));
     BB_LAUNCH_CHECK();
@@ -606,24 +799,133 @@ int blond_adjoint_spectral(int mode, const double* x, int n_slices, const double
 
 namespace bb {
 
-// The induced-voltage transform of the turn loops below: one plan and one
-// twiddle table for the whole run (the per-turn entry point builds the plan
-// on the host and the twiddles in the kernel at every call).
-struct AdjSpectral {
-    SpecPlan plan = {};
-    double2* tw = nullptr;
-    ~AdjSpectral() {
-        if (tw) cudaFree(tw);
+// Scratch of a run, ordered on its stream: no device synchronisation, and
+// calls of other threads and streams have their own.  The library's pool
+// keeps at most 64 MB of freed scratch per device and returns the rest.
+static cudaMemPool_t adj_pool() {
+    static cudaMemPool_t pool[64] = {nullptr};
+    static std::mutex mu;
+    const int dev = device_info().device;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!pool[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+        uint64_t keep = 64ull << 20;
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        pool[dev] = p;
     }
-    int init(int64_t n_fft) {
-        if (!make_spec_plan(n_fft, plan)) {
-            set_error("adjoint run: n_fft=%lld is not an even 5-smooth length <= %lld",
-                      (long long)n_fft, (long long)kMaxClusterFFT);
-            return BLOND_ERR_UNSUPPORTED;
+    return pool[dev];
+}
+
+struct AdjScratch {
+    void* p = nullptr;
+    cudaStream_t s = nullptr;
+    ~AdjScratch() {
+        if (p) cudaFreeAsync(p, s);
+    }
+    int init(size_t bytes, cudaStream_t stream) {
+        const cudaMemPool_t pool = adj_pool();
+        if (!pool) {
+            set_error("adjoint run: memory pool creation failed");
+            return BLOND_ERR_CUDA;
         }
+        s = stream;
+        BB_CUDA(cudaMallocFromPoolAsync(&p, bytes, pool, stream));
+        return BLOND_OK;
+    }
+};
+
+// The induced voltages of a run: short profiles by direct convolution
+// (convolve.cuh) -- then the spectra follow in one batched transform after
+// the turn loop -- others by one transform per turn.  One plan, twiddle table
+// and response for the whole run.
+struct AdjVoltage {
+    SpecPlan plan = {};
+    ConvPlan cplan = {};
+    bool conv = false;
+    AdjScratch mem;
+    double2* tw = nullptr;
+    double* hx = nullptr;
+    u64* raw = nullptr;      // fixed-point profile between two turns
+    int* ticket = nullptr;
+    unsigned* done = nullptr;
+    double2* rows = nullptr;  // spectra of kRows profiles
+    static constexpr int kRows = 64;
+
+    // H: the run's impedance or nullptr (then only `done` is set up)
+    int init(const double* H, int64_t n_fft, int S, cudaStream_t s) {
+        size_t tw_bytes = 0, y_bytes = 0, hx_bytes = 0, row_bytes = 0;
         int rc;
-        if ((rc = prepare_spectral())) return rc;
-        return make_spec_twiddles(plan, &tw);
+        if (H) {
+            if (!make_spec_plan(n_fft, plan)) {
+                set_error("adjoint run: n_fft=%lld is not an even 5-smooth length <= %lld",
+                          (long long)n_fft, (long long)kMaxClusterFFT);
+                return BLOND_ERR_UNSUPPORTED;
+            }
+            if ((rc = prepare_spectral())) return rc;
+            conv = n_fft >= S && make_conv_plan(S, n_fft, 1, cplan);
+            if (conv && (rc = prepare_conv())) return rc;
+            tw_bytes = (spec_twiddle_bytes(plan) + 15) & ~(size_t)15;
+            if (conv) {
+                y_bytes = 8 * ((size_t)n_fft + 1);
+                hx_bytes = 16 * (size_t)S;
+                row_bytes = 16 * (size_t)kRows * (n_fft / 2 + 1);
+            }
+        }
+        const size_t raw_bytes = (8 * (size_t)S + 15) & ~(size_t)15;
+        y_bytes = (y_bytes + 15) & ~(size_t)15;
+        if ((rc = mem.init(tw_bytes + y_bytes + hx_bytes + row_bytes + raw_bytes + 16, s)))
+            return rc;
+        char* p = static_cast<char*>(mem.p);
+        tw = reinterpret_cast<double2*>(p);
+        rows = reinterpret_cast<double2*>(p + tw_bytes);
+        double* const y = reinterpret_cast<double*>(p + tw_bytes + row_bytes);
+        hx = reinterpret_cast<double*>(p + tw_bytes + row_bytes + y_bytes);
+        raw = reinterpret_cast<u64*>(p + tw_bytes + row_bytes + y_bytes + hx_bytes);
+        ticket = reinterpret_cast<int*>(reinterpret_cast<char*>(raw) + raw_bytes);
+        done = reinterpret_cast<unsigned*>(ticket + 1);
+        BB_CUDA(cudaMemsetAsync(raw, 0, raw_bytes + 16, s));
+        if (H && (rc = fill_spec_twiddles(plan, tw, s))) return rc;
+        if (conv && (rc = conv_response_async(reinterpret_cast<const double2*>(H), n_fft, S, y,
+                                              hx, s)))
+            return rc;
+        return BLOND_OK;
+    }
+    // y = -scale h (*) x of one profile: counts, or with `deposit` the
+    // fixed-point one in `raw`, which is converted to counts and cleared
+    int convolve(const double* x, int fix_bits, double* counts, int S, double scale, double* y,
+                 cudaStream_t s) const {
+        ConvParams P = {};
+        P.p = cplan;
+        P.hx = hx;
+        P.in_f64 = x;
+        if (!x) {
+            P.in_fix = raw;
+            P.fix_unit = ldexp(1.0, -fix_bits);
+            P.profile_out = counts;
+            P.ticket = ticket;
+        }
+        P.out = y;
+        P.out_scale = -scale;
+        P.pdl = 1;
+        return launch_conv(P, s);
+    }
+    // spectra of n_rows consecutive profiles
+    int spectra(const double* x, int S, int n_rows, double* out, cudaStream_t s) const {
+        SpecParams P = {};
+        shrink_spec_plan(plan, n_rows >= 64 ? 1 : 4, P.p);
+        if (P.p.smem > device_info().max_smem_optin) P.p = plan;
+        P.twg = tw;
+        P.mode = SPEC_FORWARD | SPEC_OUT_SPECTRUM;
+        P.in_f64 = x;
+        P.n_in = S;
+        P.spec_out = reinterpret_cast<double2*>(out);
+        P.batch = n_rows;
+        return launch_spectral(P, s);
     }
     // the same transform as blond_adjoint_spectral(mode, ...)
     int run(int mode, const double* x, int S, const double* H, double scale, double* y,
@@ -652,19 +954,37 @@ struct AdjSpectral {
     }
 };
 
-// A zeroed device counter for the forward kernel's last-block conversion,
-// owned by one run.
-struct AdjCounter {
-    unsigned* p = nullptr;
-    ~AdjCounter() {
-        if (p) cudaFree(p);
+template <int PREC, int R>
+static auto adj_segment_for(int n_rf) {
+    switch (n_rf) {
+        case 0: return adj_segment_kernel<PREC, 0, R>;
+        case 1: return adj_segment_kernel<PREC, 1, R>;
+        case 2: return adj_segment_kernel<PREC, 2, R>;
+        case 3: return adj_segment_kernel<PREC, 3, R>;
+        default: return adj_segment_kernel<PREC, 4, R>;
     }
-    int init(cudaStream_t s) {
-        BB_CUDA(cudaMalloc(&p, sizeof(unsigned)));
-        BB_CUDA(cudaMemsetAsync(p, 0, sizeof(unsigned), s));
-        return BLOND_OK;
-    }
-};
+}
+
+// The turn-start coordinates of turns [0, n_sub) from dt_in, dE_in: states
+// (n_sub + 1 rows) and the final energies.
+static int launch_segment(int precision, const AdjSegment& G, const double* dt_in,
+                          const void* dE_in, double* states, void* dE_out, cudaStream_t s) {
+    // one particle a thread while that fills the SMs, else four
+    const int64_t resident = (int64_t)device_info().sm_count * 2 * kAdjSegThreads;
+    const bool one = G.T.n <= resident;
+    const auto k = precision == BLOND_PREC_F64
+                       ? (one ? adj_segment_for<BLOND_PREC_F64, 1>(G.T.n_rf)
+                              : adj_segment_for<BLOND_PREC_F64, 4>(G.T.n_rf))
+                       : (one ? adj_segment_for<BLOND_PREC_F32P64, 1>(G.T.n_rf)
+                              : adj_segment_for<BLOND_PREC_F32P64, 4>(G.T.n_rf));
+    int rc;
+    if ((rc = adj_allow_smem(k))) return rc;
+    const int grid = particle_grid(G.T.n, kAdjSegThreads, 2);
+    const size_t smem = G.vind && G.smem_vind ? 3 * sizeof(double) * (size_t)G.T.S : 0;
+    k<<<grid, kAdjSegThreads, smem, s>>>(G, dt_in, dE_in, states, dE_out);
+    BB_LAUNCH_CHECK();
+    return BLOND_OK;
+}
 
 }  // namespace bb
 
@@ -692,14 +1012,17 @@ int blond_adjoint_forward_run(int precision, double* dt, void* dE, int64_t n, in
     cudaStream_t s = as_stream(stream);
     const size_t esz = precision == BLOND_PREC_F64 ? sizeof(double) : sizeof(float);
     const int64_t M1 = n_fft / 2 + 1;
-    AdjSpectral sp;
-    AdjCounter done;
+    AdjVoltage sp;
     int rc;
-    if (impedance && (rc = sp.init(n_fft))) return rc;
-    if ((rc = done.init(s))) return rc;
-    if ((rc = blond_adjoint_deposit(dt, n, n_slices, bin_center0, inv_bin_width, profile,
-                                    stream)))
+    if ((rc = sp.init(impedance, n_fft, n_slices, s))) return rc;
+    const int bits = fixed_bits(n);
+    if (sp.conv) {
+        if ((rc = adj_deposit_launch(dt, n, n_slices, bin_center0, inv_bin_width, sp.raw, s)))
+            return rc;
+    } else if ((rc = blond_adjoint_deposit(dt, n, n_slices, bin_center0, inv_bin_width, profile,
+                                           stream))) {
         return rc;
+    }
     for (int64_t t = 0; t < n_turns; ++t) {
         if (t % checkpoint_every == 0) {
             const int64_t seg = t / checkpoint_every;
@@ -709,16 +1032,31 @@ int blond_adjoint_forward_run(int precision, double* dt, void* dE, int64_t n, in
                                     esz * n, cudaMemcpyDeviceToDevice, s));
         }
         double* vind = impedance ? induced_voltage + t * n_slices : nullptr;
-        if (impedance &&
-            (rc = sp.run(0, profile + t * n_slices, n_slices, impedance, scale, vind,
-                         spectrum + t * M1 * 2, nullptr, s)))
-            return rc;
+        double* const next = profile + (t + 1) * n_slices;
+        if (sp.conv)
+            rc = sp.convolve(nullptr, bits, profile + t * n_slices, n_slices, scale, vind, s);
+        else if (impedance)
+            rc = sp.run(0, profile + t * n_slices, n_slices, impedance, scale, vind,
+                        spectrum + t * M1 * 2, nullptr, s);
+        if (rc) return rc;
+        // (with the convolution the next turn's launch converts the deposit)
         if ((rc = adj_forward_launch(
                  precision, dt, dE, dt, dE, n, n_rf, voltage + t * n_rf, omega_rf + t * n_rf,
                  phi_rf + t * n_rf, acc_kick[t], charge, drift_coeff[t], vind, n_slices,
-                 bin_center0, inv_bin_width, profile + (t + 1) * n_slices, done.p, stream,
-                 true)))
+                 bin_center0, inv_bin_width, sp.conv ? reinterpret_cast<double*>(sp.raw) : next,
+                 sp.conv ? nullptr : sp.done, stream, true, sp.conv)))
             return rc;
+    }
+    if (sp.conv) {
+        fixed_to_counts_from_kernel<<<(n_slices + 255) / 256, 256, 0, s>>>(
+            sp.raw, profile + n_turns * n_slices, n_slices, bits);
+        BB_LAUNCH_CHECK();
+        // the spectra of the turns' profiles, in launches of at most 4096
+        for (int64_t t = 0; t < n_turns; t += 4096)
+            if ((rc = sp.spectra(profile + t * n_slices, n_slices,
+                                 (int)std::min<int64_t>(4096, n_turns - t),
+                                 spectrum + t * M1 * 2, s)))
+                return rc;
     }
     return BLOND_OK;
 }
@@ -752,24 +1090,38 @@ int blond_adjoint_backward_run(int precision, int64_t n, int n_rf, int64_t n_tur
     const int64_t K = checkpoint_every;
     const int64_t nseg = (n_turns + K - 1) / K;
     const bool has_z = impedance_conj != nullptr;
-    AdjSpectral sp;
+    AdjVoltage sp;
     int rc;
-    if (has_z && (rc = sp.init(n_fft))) return rc;
+    if (has_z && (rc = sp.init(impedance_conj, n_fft, n_slices, s))) return rc;
     const double* lam_p = lam_p_final;
     for (int64_t seg = nseg - 1; seg >= 0; --seg) {
         const int64_t a = seg * K, b = std::min(n_turns, (seg + 1) * K);
         // the segment's turn-start coordinates, recomputed from its checkpoint
-        BB_CUDA(cudaMemcpyAsync(states, ckpt_dt + seg * n, sizeof(double) * n,
-                                cudaMemcpyDeviceToDevice, s));
-        BB_CUDA(cudaMemcpyAsync(dE_work, static_cast<const char*>(ckpt_dE) + (size_t)seg * n * esz,
-                                esz * n, cudaMemcpyDeviceToDevice, s));
-        for (int64_t t = a; t < b; ++t) {
-            if ((rc = adj_forward_launch(
-                     precision, states + (t - a) * n, dE_work, states + (t - a + 1) * n,
-                     dE_work, n, n_rf, voltage + t * n_rf, omega_rf + t * n_rf,
-                     phi_rf + t * n_rf, acc_kick[t], charge, drift_coeff[t],
-                     has_z ? induced_voltage + t * n_slices : nullptr, n_slices, bin_center0,
-                     inv_bin_width, nullptr, nullptr, stream, true)))
+        for (int64_t t = a; t < b; t += kAdjSegTurns) {
+            AdjSegment G = {};
+            G.T.n = n;
+            G.T.n_rf = n_rf;
+            G.T.V = voltage + t * n_rf;
+            G.T.om = omega_rf + t * n_rf;
+            G.T.ph = phi_rf + t * n_rf;
+            G.T.charge = charge;
+            G.T.S = n_slices;
+            G.T.bc0 = bin_center0;
+            G.T.inv_w = inv_bin_width;
+            G.n_sub = (int)std::min<int64_t>(kAdjSegTurns, b - t);
+            G.vind = has_z ? induced_voltage + t * n_slices : nullptr;
+            G.smem_vind = 3 * sizeof(double) * n_slices <= kAdjSegSmem;
+            for (int q = 0; q < G.n_sub; ++q) {
+                G.acc[q] = acc_kick[t + q];
+                G.drift_c[q] = drift_coeff[t + q];
+            }
+            const bool first = t == a;
+            if ((rc = launch_segment(
+                     precision, G, first ? ckpt_dt + seg * n : states + (t - a) * n,
+                     first ? static_cast<const void*>(static_cast<const char*>(ckpt_dE) +
+                                                      (size_t)seg * n * esz)
+                           : dE_work,
+                     states + (t - a) * n, dE_work, s)))
                 return rc;
         }
         for (int64_t t = b - 1; t >= a; --t) {
@@ -782,14 +1134,30 @@ int blond_adjoint_backward_run(int precision, int64_t n, int n_rf, int64_t n_tur
                      true)))
                 return rc;
             if (has_z) {
-                if ((rc = sp.run(1, lam_v + t * n_slices, n_slices, impedance_conj, scale,
-                                 lam_pt + t * n_slices, const_cast<double*>(spectrum) + t * M1 * 2,
-                                 spectrum_accum, s)))
-                    return rc;
+                if (sp.conv)
+                    rc = sp.convolve(lam_v + t * n_slices, 0, nullptr, n_slices, scale,
+                                     lam_pt + t * n_slices, s);
+                else
+                    rc = sp.run(1, lam_v + t * n_slices, n_slices, impedance_conj, scale,
+                                lam_pt + t * n_slices,
+                                const_cast<double*>(spectrum) + t * M1 * 2, spectrum_accum, s);
+                if (rc) return rc;
                 lam_p = lam_pt + t * n_slices;
             } else {
                 lam_p = nullptr;
             }
+        }
+        // the impedance's gradient from the segment's spectra
+        for (int64_t hi = b; sp.conv && hi > a; hi -= AdjVoltage::kRows) {
+            const int64_t lo = std::max(a, hi - AdjVoltage::kRows);
+            const int rows = (int)(hi - lo);
+            if ((rc = sp.spectra(lam_v + lo * n_slices, n_slices, rows,
+                                 reinterpret_cast<double*>(sp.rows), s)))
+                return rc;
+            adj_accumulate_kernel<<<(int)((M1 + 127) / 128), 128, 0, s>>>(
+                reinterpret_cast<const double2*>(spectrum) + lo * M1, sp.rows, M1, rows,
+                reinterpret_cast<double2*>(spectrum_accum));
+            BB_LAUNCH_CHECK();
         }
     }
     // the turn-0 profile is a deposit of the initial dt

@@ -25,20 +25,25 @@ __device__ __forceinline__ void fill_shared(double* dst, int n, int tid, int nth
 // next bin needs the same ones moved by one, so a step is two shared loads
 // (one new response value, one bin) for kConvTile multiply-adds.  A segment
 // has an odd length, so the 32 segments of a warp fall on different banks.
+//
+// One more warp takes what the outputs do not wait for: the converted
+// profile, the beam-phase sums, the ticket that tells when every block has
+// read the histogram, then (last block) the clearing and the loop's turn.  On
+// a computing warp the ticket's round trip alone took 0.7 us of a 4 us launch.
 template <bool FB>
-__global__ void __launch_bounds__(kConvThreads)
+__global__ void __launch_bounds__(kConvThreads + 32)
 conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
     pdl_launch_dependents();
     extern __shared__ double csm[];
     __shared__ double red[kConvThreads / 32][kConvTile];
     __shared__ double vs[kConvTile * kConvMaxGroups];
-    __shared__ int last;
     const int S = P.p.S, g = P.p.groups, L = P.p.seg, wpg = P.p.wpg;
     const int T = 32 * wpg * L, nth = 32 * wpg * g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int beam = P.batch ? (int)blockIdx.x / P.p.ctas : 0;
     const int cta = (int)blockIdx.x - beam * P.p.ctas;
     const int i0 = cta * P.p.chunk;
+    const int n_own = min(P.p.chunk, S - i0);
     const int64_t boff = (int64_t)beam * S;
     double* const prof = csm;     // T bins, zero beyond S
     double* const hw = csm + T;   // the responses of this block's outputs
@@ -46,7 +51,7 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
 
     // hw[q] multiplies bin j of output i0 + o at q = o - j + T - 1
     const double* const hx = P.hx + (int64_t)beam * (2 * S - 1);
-    fill_shared(hw, nh, tid, nth, [&](int q) {
+    fill_shared(hw, nh, tid, nth + 32, [&](int q) {
         const int x = i0 + q - (T - S);
         return x >= 0 && x < 2 * S - 1 ? __ldg(hx + x) : 0.0;
     });
@@ -54,22 +59,27 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
     const long long turn = P.turn ? *P.turn : 0;
     if (P.in_i32) {
         const int* const in = P.in_i32 + boff;
-        fill_shared(prof, T, tid, nth, [&](int j) { return j < S ? __ldcg(in + j) : 0; });
+        fill_shared(prof, T, tid, nth + 32, [&](int j) { return j < S ? __ldcg(in + j) : 0; });
+    } else if (P.in_fix) {
+        const unsigned long long* const in = P.in_fix + boff;
+        fill_shared(prof, T, tid, nth + 32, [&](int j) {
+            return j < S ? (double)__ldcg(in + j) * P.fix_unit : 0.0;
+        });
     } else {
         const double* const in = P.in_f64 + boff;
-        fill_shared(prof, T, tid, nth, [&](int j) { return j < S ? __ldcg(in + j) : 0.0; });
+        fill_shared(prof, T, tid, nth + 32, [&](int j) { return j < S ? __ldcg(in + j) : 0.0; });
     }
     __syncthreads();
-    bool fb_on = false;
-    if constexpr (FB) {
-        // this block's bins of the beam-phase sums
-        fb_on = turn >= fb.delay;
-        if (warp == 0) {
+    if (tid >= nth) {
+        if (P.profile_out)
+            for (int o = lane; o < n_own; o += 32) P.profile_out[boff + i0 + o] = prof[i0 + o];
+        if (!P.ticket) return;
+        if constexpr (FB) {
+            // this block's bins of the beam-phase sums
             double s = 0.0, c = 0.0;
-            if (fb_on) {
+            if (turn >= fb.delay) {
                 const FbBins b = fb_bins(fb, turn);
-                for (int o = lane; o < P.p.chunk && i0 + o < S; o += 32)
-                    fb_add(b, i0 + o, prof[i0 + o], s, c);
+                for (int o = lane; o < n_own; o += 32) fb_add(b, i0 + o, prof[i0 + o], s, c);
             }
             for (int d = 16; d > 0; d >>= 1) {
                 s += __shfl_down_sync(0xffffffffu, s, d);
@@ -80,16 +90,36 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
                 fb.phase_partials[2 * cta + 1] = c;
             }
         }
-    }
-    // every block takes a ticket once it has read the histogram and the
-    // counter; the one that takes the last clears them (no block waits)
-    if (tid == 0) {
+        int last = 0;
+        if (lane == 0) {
+            __threadfence();
+            last = atomicAdd(P.ticket + beam, 1) == P.p.ctas - 1;
+        }
+        if (!__shfl_sync(0xffffffffu, last, 0)) return;
         __threadfence();
-        last = atomicAdd(P.ticket + beam, 1) == P.p.ctas - 1;
+        // every block has read the histogram and the counter
+        if (P.in_i32)
+            for (int j = lane; j < S; j += 32) P.in_i32[boff + j] = 0;
+        if (P.in_fix)
+            for (int j = lane; j < S; j += 32) P.in_fix[boff + j] = 0ull;
+        if (lane == 0) {
+            P.ticket[beam] = 0;
+            if (P.turn && beam == 0) *P.turn = turn + 1;
+        }
+        if constexpr (FB) {
+            double s = 0.0, c = 0.0;
+            for (int q = lane; q < P.p.ctas; q += 32) {
+                s += __ldcg(fb.phase_partials + 2 * q);
+                c += __ldcg(fb.phase_partials + 2 * q + 1);
+            }
+            for (int d = 16; d > 0; d >>= 1) {
+                s += __shfl_down_sync(0xffffffffu, s, d);
+                c += __shfl_down_sync(0xffffffffu, c, d);
+            }
+            if (lane == 0) fb_turn_end(fb, turn, s, c, 0.0);
+        }
+        return;
     }
-    if (P.in_i32 && P.profile_out)
-        for (int o = tid; o < P.p.chunk && i0 + o < S; o += nth)
-            P.profile_out[boff + i0 + o] = prof[i0 + o];
 
     const int grp = warp / wpg, seg = (warp - grp * wpg) * 32 + lane;
     const double* const pj = prof + seg * L;
@@ -131,9 +161,10 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
     acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
     acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
     if ((lane & 3) == 0) red[warp][lane >> 2] = acc[0];
-    __syncthreads();
+    // the computing warps' barrier
+    auto compute_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(nth) : "memory"); };
+    compute_sync();
 
-    const int n_own = min(P.p.chunk, S - i0);
     if (tid < kConvTile * g) {
         double v = 0.0;
         for (int q = 0; q < wpg; ++q) v += red[(tid / kConvTile) * wpg + q][tid % kConvTile];
@@ -162,7 +193,7 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
         vs[tid] = v;
     }
     if (P.table) {
-        __syncthreads();
+        compute_sync();
         if (tid < n_own && i0 + tid < S - 1) {
             const int n = i0 + tid;
             const double a0 = vs[tid], a1 = vs[tid + 1];
@@ -187,28 +218,6 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
             }
         }
     }
-    if (!last) return;  // written before the first barrier after the ticket
-    if (P.in_i32)
-        for (int j = tid; j < S; j += nth) P.in_i32[boff + j] = 0;
-    if (tid == 0) {
-        P.ticket[beam] = 0;
-        if (P.turn && beam == 0) *P.turn = turn + 1;
-    }
-    if constexpr (FB) {
-        if (warp == 0) {
-            __threadfence();
-            double s = 0.0, c = 0.0;
-            for (int q = lane; q < P.p.ctas; q += 32) {
-                s += __ldcg(fb.phase_partials + 2 * q);
-                c += __ldcg(fb.phase_partials + 2 * q + 1);
-            }
-            for (int d = 16; d > 0; d >>= 1) {
-                s += __shfl_down_sync(0xffffffffu, s, d);
-                c += __shfl_down_sync(0xffffffffu, c, d);
-            }
-            if (lane == 0) fb_turn_end(fb, turn, s, c, 0.0);
-        }
-    }
 }
 
 bool make_conv_plan(int S, int64_t N, int B, ConvPlan& plan) {
@@ -221,9 +230,10 @@ bool make_conv_plan(int S, int64_t N, int B, ConvPlan& plan) {
     // 12.8 -> 14.2, 9000 61.6 -> 16.7)
     if (B == 1 && pow2 && S > 4600) return false;
     // a batch: the profiles' multiply-adds share the SMs (37 beams of 400
-    // slices 21.2 -> 15.4 us a turn, but 256 of 512 would be 26.8 -> 29);
-    // up to 8 beams take the single beam's rule, so that they also take its bits
-    if (B > 1 && (int64_t)B * S * S > 30'000'000 && (B > 8 || S > 4600)) return false;
+    // slices 21.2 -> 14.5 us a turn, but 64 of 512 would be 16 -> 23 and 256 of
+    // 300 37 -> 40); up to 8 beams take the single beam's rule, so that they
+    // also take its bits
+    if (B > 1 && (int64_t)B * S * S > 8'000'000 && (B > 8 || S > 4600)) return false;
     int g = 1;
     while (g < kConvMaxGroups && (kConvTile * g - 1) * sms < S) ++g;
     if ((kConvTile * g - 1) * sms < S) return false;
@@ -283,6 +293,15 @@ int make_conv_response(const double2* H, int64_t N, int S, int B, double** hx) {
     return rc;
 }
 
+int conv_response_async(const double2* H, int64_t N, int S, double* y, double* hx,
+                        cudaStream_t stream) {
+    const int rc = blond_irfft_f64(reinterpret_cast<const double*>(H), N, y, N, stream);
+    if (rc) return rc;
+    conv_response_kernel<<<dim3((2 * S + 254) / 256, 1), 256, 0, stream>>>(y, N, S, hx);
+    BB_LAUNCH_CHECK();
+    return BLOND_OK;
+}
+
 int prepare_conv() {
     static bool done[64] = {false};
     const DeviceInfo& d = device_info();
@@ -305,7 +324,7 @@ static int launch_conv_t(const ConvParams& P, const typename ConvLoopArg<FB>::ty
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.p.ctas * (P.batch > 0 ? P.batch : 1));
-    cfg.blockDim = dim3(32 * P.p.wpg * P.p.groups);
+    cfg.blockDim = dim3(32 * P.p.wpg * P.p.groups + 32);
     cfg.dynamicSmemBytes = P.p.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -22,7 +22,8 @@
 
 namespace bb {
 
-constexpr int kConvThreads = 512;   // at most
+constexpr int kConvThreads = 512;   // computing threads, at most; one more warp
+                                    // clears up and runs the loop
 constexpr int kConvTile = 8;        // outputs a thread accumulates in registers
 constexpr int kConvMaxGroups = 12;  // tiles of outputs per block
 
@@ -40,11 +41,14 @@ struct ConvParams {
     ConvPlan p;
     // the impulse response around 0: hx[B][2 S - 1], hx[x] = h_{(x - (S-1)) mod N}
     const double* hx;
-    // the profile: exactly one of in_f64 / in_i32 (the engine's histogram,
-    // zeroed by the last block to have read it)
+    // the profile: exactly one of in_f64, in_i32 (the engine's histogram) and
+    // in_fix (the adjoint's fixed-point deposit, 2^fix_bits units a particle);
+    // the last two are zeroed by the last block to have read them
     const double* in_f64;
     int* in_i32;
-    double* profile_out;      // the converted histogram
+    unsigned long long* in_fix;
+    double fix_unit;          // 2^-fix_bits
+    double* profile_out;      // the converted histogram or deposit
     double* out;              // the induced voltage
     double out_scale;
     const double* beam_scale; // batch: per profile, in place of out_scale
@@ -67,7 +71,8 @@ struct ConvParams {
     int n_rf;
     long long n_turns;
     long long* turn;          // device turn counter, advanced once
-    int* ticket;              // one per profile, zero between launches
+    int* ticket;              // one per profile, zero between launches (in_i32,
+                              // in_fix, turn or a loop need it)
     int batch;                // profiles (0: one)
     int pdl;
 };
@@ -82,6 +87,9 @@ bool make_conv_plan(int S, int64_t N, int B, ConvPlan& plan);
 // hx (cudaMalloc'd, B (2 S - 1) doubles) from the impedances H, B x (N/2 + 1)
 // values on the device.  Synchronous.
 int make_conv_response(const double2* H, int64_t N, int S, int B, double** hx);
+// The same on a stream into caller memory: hx and y (N doubles of scratch).
+int conv_response_async(const double2* H, int64_t N, int S, double* y, double* hx,
+                        cudaStream_t stream);
 // Kernel attributes, set outside stream capture.
 int prepare_conv();
 int launch_conv(const ConvParams& P, cudaStream_t stream);

@@ -153,13 +153,22 @@ __global__ void twiddle_table_kernel(const SpecPlan p, double2* out) {
                   at(lay.tbn), threadIdx.x, blockDim.x);
 }
 
-int make_spec_twiddles(const SpecPlan& plan, double2** out) {
+size_t spec_twiddle_bytes(const SpecPlan& plan) {
     const SpecLayout lay = spec_layout(plan);
-    const size_t bytes = (size_t)(lay.hk - lay.tw1);
-    *out = nullptr;
-    BB_CUDA(cudaMalloc(out, bytes));
-    twiddle_table_kernel<<<1, 512>>>(plan, *out);
+    return (size_t)(lay.hk - lay.tw1);
+}
+
+int fill_spec_twiddles(const SpecPlan& plan, double2* out, cudaStream_t stream) {
+    twiddle_table_kernel<<<1, 512, 0, stream>>>(plan, out);
     BB_LAUNCH_CHECK();
+    return BLOND_OK;
+}
+
+int make_spec_twiddles(const SpecPlan& plan, double2** out) {
+    *out = nullptr;
+    BB_CUDA(cudaMalloc(out, spec_twiddle_bytes(plan)));
+    const int rc = fill_spec_twiddles(plan, *out, nullptr);
+    if (rc) return rc;
     BB_CUDA(cudaDeviceSynchronize());
     return BLOND_OK;
 }

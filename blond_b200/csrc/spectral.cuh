@@ -104,8 +104,9 @@ struct SpecParams {
     // batch of independent profiles: cluster q (blockIdx.x / C) handles
     // profile q; in_i32 / profile_out / out / bc / table advance by n_in
     // entries per profile, H by M + 1; beam_scale[q] and beam_inv_w[q]
-    // replace out_scale and inv_w when given.  No inductive term and no
-    // turn reads in batch mode (only the last cluster bumps the counter).
+    // replace out_scale and inv_w when given; spec_out advances by M + 1.  No
+    // inductive term and no turn reads in batch mode (only the last cluster
+    // bumps the counter).
     int batch;
     const double* beam_scale;
     const double* beam_inv_w;
@@ -499,6 +500,7 @@ spectral_kernel(const SpecParams P, const typename SpecLoopArg<FB>::type LP) {
     void* const g_table =
         P.table ? static_cast<char*>(P.table) + boff * (P.table_f32 ? 8 : 16) : nullptr;
     const double2* const g_H = P.H ? P.H + (int64_t)beam * (M + 1) : nullptr;
+    double2* const g_spec = P.spec_out ? P.spec_out + (int64_t)beam * (M + 1) : nullptr;
     const double out_scale = P.beam_scale ? P.beam_scale[beam] : P.out_scale;
     const double inv_w = P.beam_inv_w ? P.beam_inv_w[beam] : P.inv_w;
     double2* buf[3] = {reinterpret_cast<double2*>(sraw + lay.bufs),
@@ -717,8 +719,8 @@ spectral_kernel(const SpecParams P, const typename SpecLoopArg<FB>::type LP) {
                 }
                 if (P.mode & SPEC_OUT_SPECTRUM) {
                     // every k < M is owned once; X[M] comes from k == 0
-                    P.spec_out[k] = Yk;
-                    if (k == 0) P.spec_out[M] = Yp;
+                    g_spec[k] = Yk;
+                    if (k == 0) g_spec[M] = Yp;
                 }
                 if (P.mode & SPEC_ACCUM) {
                     P.acc_g[k] = cadd(P.acc_g[k], cmul(P.acc_a[k], cconj(Yk)));
@@ -918,5 +920,8 @@ int prepare_spectral();
 // Allocate (cudaMalloc) and fill the twiddle tables of a plan for
 // SpecParams::twg; the caller frees *out with cudaFree.  Synchronous.
 int make_spec_twiddles(const SpecPlan& plan, double2** out);
+// The same on a stream into caller memory of spec_twiddle_bytes(plan).
+size_t spec_twiddle_bytes(const SpecPlan& plan);
+int fill_spec_twiddles(const SpecPlan& plan, double2* out, cudaStream_t stream);
 
 }  // namespace bb
