@@ -56,10 +56,19 @@ static int histogram_smem_budget() {
 }
 
 constexpr int kThreads = 512;
+// Particles per thread and iteration of the streaming kernels: their loads
+// go out together, so that 64 KB and more per SM are in flight (one load per
+// thread left 8 to 16 KB, latency-bound at half of the HBM rate).
+constexpr int kUnroll = 4;
+// ... where there are that many for every resident thread; below, one each
+// keeps all threads busy (3e5 particles: kick 3.1 us, 6.7 with four).
+static bool unroll_pays(int64_t n) {
+    return n >= (int64_t)kUnroll * 4 * kThreads * device_info().sm_count;
+}
 constexpr int kMaxRf = 64;
 
 // ------------------------------------------------------------ RF kick
-template <typename T>
+template <typename T, int U>
 __global__ void __launch_bounds__(kThreads)
 kick_kernel(const T* __restrict__ dt, T* __restrict__ dE, int n_rf, T charge,
             const T* __restrict__ voltage, const T* __restrict__ omega,
@@ -71,13 +80,26 @@ kick_kernel(const T* __restrict__ dt, T* __restrict__ dE, int n_rf, T charge,
         sp[j] = phi[j];
     }
     __syncthreads();
+    // U particles a thread, all loads issued before any arithmetic
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += stride) {
-        const T t = dt[i];
-        T s = 0;
-        for (int j = 0; j < n_rf; ++j) s += sv[j] * dev_sin(so[j] * t + sp[j]);
-        dE[i] += charge * s + acc;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n;
+         i0 += U * stride) {
+        T t[U], e[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = i0 + u * stride;
+            t[u] = i < n ? dt[i] : T(0);
+            e[u] = i < n ? dE[i] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            T s = 0;
+            for (int j = 0; j < n_rf; ++j) s += sv[j] * dev_sin(so[j] * t[u] + sp[j]);
+            e[u] += charge * s + acc;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + u * stride < n) dE[i0 + u * stride] = e[u];
     }
 }
 
@@ -92,8 +114,11 @@ static int kick_impl(const T* dt, T* dE, int n_rf, T charge, const T* V,
     BB_CHECK_ARG(dt && dE, "kick: null particle array");
     BB_CHECK_ARG(n_rf == 0 || (V && om && ph), "kick: null RF array");
     const int grid = particle_grid(n, kThreads, 4);
-    kick_kernel<T><<<grid, kThreads, 0, as_stream(stream)>>>(
-        dt, dE, n_rf, charge, V, om, ph, n, acc);
+    // (sinf's branches keep several sines of a thread from overlapping:
+    // float32 at two RF systems stays with one particle a thread)
+    auto k = unroll_pays(n / 2) && (sizeof(T) == 8 || n_rf <= 1) ? kick_kernel<T, kUnroll>
+                                                                 : kick_kernel<T, 1>;
+    k<<<grid, kThreads, 0, as_stream(stream)>>>(dt, dE, n_rf, charge, V, om, ph, n, acc);
     BB_LAUNCH_CHECK();
     return BLOND_OK;
 }
@@ -205,28 +230,31 @@ __device__ __forceinline__ int slice_bin(T x, T cut_left, T inv_w, int S) {
     return (f >= T(0) && f < T(S)) ? (int)f : -1;
 }
 
-// Shared-memory-privatised integer histogram.  With WARP_AGG the lanes of a
-// warp that hit the same bin are merged by __match_any_sync so one lane adds
-// the popcount -- worthwhile when few bins take most particles.
-template <typename T, bool WARP_AGG>
-__global__ void __launch_bounds__(kThreads)
+// Shared-memory-privatised integer histogram, U coordinates of a thread in
+// flight.  (Merging a warp's equal bins by __match_any_sync costs more than
+// the bank conflicts it saves from 30 slices on: 1e7 particles, 1000 slices
+// 83 us, 40 without.)  Bound: HBM reads (8 B a particle) and the flush, S
+// float additions per block -- so profiles beyond 32 KB take one block per SM.
+template <typename T, int U, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 histogram_smem_kernel(const T* __restrict__ dt, T* __restrict__ out,
                       T cut_left, T inv_w, int S, int64_t n) {
     extern __shared__ int sh[];
     for (int k = threadIdx.x; k < S; k += blockDim.x) sh[k] = 0;
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    // whole warps iterate together so __match_any_sync sees all 32 lanes
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-         base < n; base += stride) {
-        const int64_t i = base + lane;
-        const int b = i < n ? slice_bin<T>(dt[i], cut_left, inv_w, S) : -1;
-        if (WARP_AGG) {
-            const unsigned peers = __match_any_sync(0xffffffffu, b);
-            if (b >= 0 && lane == __ffs(peers) - 1) atomicAdd(&sh[b], __popc(peers));
-        } else if (b >= 0) {
-            atomicAdd(&sh[b], 1);
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n;
+         i0 += U * stride) {
+        T t[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = i0 + u * stride;
+            t[u] = i < n ? dt[i] : (T)NAN;  // beyond the beam: no slice
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int b = slice_bin<T>(t[u], cut_left, inv_w, S);
+            if (b >= 0) atomicAdd(&sh[b], 1);
         }
     }
     __syncthreads();
@@ -264,22 +292,19 @@ static int histogram_impl(const T* dt, T* out, T cut_left, T cut_right,
     const T inv_w = (T)S / (cut_right - cut_left);
     const size_t smem = sizeof(int) * (size_t)S;
     if ((int64_t)smem <= histogram_smem_budget()) {
-        // one or two resident blocks per SM depending on the table size
-        const int per_sm = smem <= 96 * 1024 ? 2 : 1;
-        const int grid = particle_grid(n, kThreads, per_sm);
-        if (S <= 2048) {
-            BB_CUDA(cudaFuncSetAttribute(histogram_smem_kernel<T, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-            histogram_smem_kernel<T, true><<<grid, kThreads, smem, s>>>(dt, out, cut_left,
-                                                                        inv_w, S, n);
-        } else {
-            BB_CUDA(cudaFuncSetAttribute(histogram_smem_kernel<T, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-            histogram_smem_kernel<T, false><<<grid, kThreads, smem, s>>>(dt, out, cut_left,
-                                                                         inv_w, S, n);
-        }
+        auto launch = [&](auto k, int threads, int per_sm) {
+            const cudaError_t rc = cudaFuncSetAttribute(
+                k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (rc != cudaSuccess) return rc;
+            k<<<particle_grid(n, threads, per_sm), threads, smem, s>>>(dt, out, cut_left, inv_w,
+                                                                       S, n);
+            return cudaSuccess;
+        };
+        BB_CUDA(smem > 32 * 1024
+                    ? (unroll_pays(n) ? launch(histogram_smem_kernel<T, 8, 1024>, 1024, 1)
+                                      : launch(histogram_smem_kernel<T, 1, 1024>, 1024, 1))
+                    : (unroll_pays(n) ? launch(histogram_smem_kernel<T, 8, kThreads>, kThreads, 2)
+                                      : launch(histogram_smem_kernel<T, 1, kThreads>, kThreads, 2)));
     } else {
         const int grid = particle_grid(n, 256, 8);
         histogram_global_kernel<T><<<grid, 256, 0, s>>>(dt, out, cut_left, inv_w, S, n);
@@ -351,6 +376,13 @@ static int smooth_histogram_impl(const T* dt, T* out, T cut_left, T cut_right,
 // reference's table are recomputed at the gathered slice with the same
 // expressions, so no table buffer is needed.
 template <typename T>
+__device__ __forceinline__ T lik_value(T t, T v0, T v1, T b, T charge, T inv_w, T acc) {
+    const T slope = charge * (v1 - v0) * inv_w;
+    const T offset = (charge * v0 - b * slope) + acc;
+    return t * slope + offset;
+}
+
+template <typename T>
 __global__ void __launch_bounds__(kThreads)
 lik_kernel(const T* __restrict__ dt, T* __restrict__ dE,
            const T* __restrict__ V, const T* __restrict__ bc, T charge, int S,
@@ -364,10 +396,48 @@ lik_kernel(const T* __restrict__ dt, T* __restrict__ dE,
         const T f = dev_floor((t - bc0) * inv_w);
         if (!(f >= T(0) && f < T(S - 1))) continue;
         const int k = (int)f;
-        const T v0 = __ldg(V + k), v1 = __ldg(V + k + 1);
-        const T slope = charge * (v1 - v0) * inv_w;
-        const T offset = (charge * v0 - __ldg(bc + k) * slope) + acc;
-        dE[i] += t * slope + offset;
+        dE[i] += lik_value(t, __ldg(V + k), __ldg(V + k + 1), __ldg(bc + k), charge, inv_w, acc);
+    }
+}
+
+// The same for large beams with the voltages (BC: and the bin centres) in
+// shared memory, kUnroll particles a thread in flight: three gathers through
+// L1 per particle bound the pass above at 58 us for 1e7 float64 particles
+// (36.6 us of HBM time).
+constexpr int kLikThreads = 1024;
+template <typename T, bool BC>
+__global__ void __launch_bounds__(kLikThreads, 1)
+lik_smem_kernel(const T* __restrict__ dt, T* __restrict__ dE, const T* __restrict__ V,
+                const T* __restrict__ bc, T charge, int S, int64_t n, T acc) {
+    extern __shared__ __align__(16) unsigned char lsm[];
+    T* const sv = reinterpret_cast<T*>(lsm);
+    T* const sb = sv + S;
+    const T bc0 = bc[0];
+    const T inv_w = (T)(S - 1) / (bc[S - 1] - bc0);
+#pragma unroll 4
+    for (int k = threadIdx.x; k < S; k += blockDim.x) {
+        sv[k] = V[k];
+        if (BC) sb[k] = bc[k];
+    }
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n;
+         i0 += kUnroll * stride) {
+        T t[kUnroll], e[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int64_t i = i0 + u * stride;
+            t[u] = i < n ? dt[i] : (T)NAN;  // beyond the beam: no slice
+            e[u] = i < n ? dE[i] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const T f = dev_floor((t[u] - bc0) * inv_w);
+            if (!(f >= T(0) && f < T(S - 1))) continue;
+            const int k = (int)f;
+            dE[i0 + u * stride] = e[u] + lik_value(t[u], sv[k], sv[k + 1],
+                                                   BC ? sb[k] : __ldg(bc + k), charge, inv_w, acc);
+        }
     }
 }
 
@@ -378,9 +448,22 @@ static int lik_impl(const T* dt, T* dE, const T* V, const T* bc, T charge,
     BB_CHECK_SIZE(S >= 2, "linear_interp_kick: n_slices=%d must be >= 2", S);
     if (n == 0) return BLOND_OK;
     BB_CHECK_ARG(dt && dE && V && bc, "linear_interp_kick: null pointer");
-    const int grid = particle_grid(n, kThreads, 4);
-    lik_kernel<T><<<grid, kThreads, 0, as_stream(stream)>>>(dt, dE, V, bc, charge, S,
-                                                            n, acc);
+    cudaStream_t s = as_stream(stream);
+    // shared-memory tables where a block's particles outweigh their copy
+    // (float64, 16384 slices: 2e6 particles 21.5 us without and 25.6 with
+    // them, 3e7 160 and 144)
+    const size_t table = sizeof(T) * (size_t)S, room = (size_t)histogram_smem_budget();
+    if (unroll_pays(n) && n >= (int64_t)400 * S && table <= room) {
+        const bool both = 2 * table <= room;
+        auto k = both ? lik_smem_kernel<T, true> : lik_smem_kernel<T, false>;
+        const int smem = (int)(both ? 2 * table : table);
+        BB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k<<<particle_grid(n, kLikThreads, 1), kLikThreads, smem, s>>>(dt, dE, V, bc, charge, S, n,
+                                                                      acc);
+    } else {
+        lik_kernel<T><<<particle_grid(n, kThreads, 4), kThreads, 0, s>>>(dt, dE, V, bc, charge, S,
+                                                                         n, acc);
+    }
     BB_LAUNCH_CHECK();
     return BLOND_OK;
 }
