@@ -3,6 +3,7 @@
 // lengths the cluster transform does not take (odd, or prime factors > 5).
 #define BB_SPECTRAL_KERNELS
 #include "spectral.cuh"
+#include "head_fft.cuh"
 
 #include <vector>
 
@@ -99,6 +100,8 @@ int prepare_spectral() {
         BB_CUDA(cudaFuncSetAttribute(spectral_kernel<true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      d.max_smem_optin));
+        const int rc = prepare_head_fft();
+        if (rc) return rc;
         attr_done[d.device & 63] = true;
     }
     return BLOND_OK;
@@ -134,6 +137,7 @@ static int launch_spectral_t(const SpecParams& P, const typename SpecLoopArg<FB>
 }
 
 int launch_spectral(const SpecParams& P, cudaStream_t stream) {
+    if (head_fft_takes(P)) return launch_head_fft(P, stream);
     return launch_spectral_t<false>(P, SpecNoLoop{}, stream);
 }
 

@@ -251,7 +251,7 @@ __device__ __forceinline__ void small_dft(double2* v, int R, double s) {
 // Index arithmetic avoids integer division when the batch count B and the
 // stride Ns are powers of two (lgB / lgNs >= 0): every power-of-two length,
 // i.e. every next_regular result of the usual 2^k slice counts.
-__device__ __noinline__ void stockham_pass(const double2* __restrict__ src,
+static __device__ __noinline__ void stockham_pass(const double2* __restrict__ src,
                                            double2* __restrict__ dst, int L, int B,
                                            int Ns, int R, const double2* __restrict__ tw,
                                            double s, int lgB, int lgNs, int LR, int step) {
@@ -378,7 +378,7 @@ __device__ __forceinline__ void subwarp_fft(double2* a, int B, const double2* __
 // head calls the transform batch six times, and six inlined copies of these
 // made the kernel's code about 700 KB, whose instruction fetches were the
 // head's top stall.
-__device__ __noinline__ void warp_fft_any(double2* a, int L, int B, const double2* tw,
+static __device__ __noinline__ void warp_fft_any(double2* a, int L, int B, const double2* tw,
                                           bool inverse) {
     switch (L) {
         case 2: subwarp_fft<2>(a, B, tw, inverse, 1); return;
@@ -394,7 +394,7 @@ __device__ __noinline__ void warp_fft_any(double2* a, int L, int B, const double
 
 // B transforms of length L, interleaved, starting in a[]; returns the buffer
 // (a or b) that holds the result.  Ends with __syncthreads().
-__device__ double2* batch_fft(double2* a, double2* b, int L, int B, const int* radices,
+static __device__ double2* batch_fft(double2* a, double2* b, int L, int B, const int* radices,
                               int npass, const double2* tw, bool inverse) {
     if (L >= 2 && L <= 256 && (L & (L - 1)) == 0) {
         warp_fft_any(a, L, B, tw, inverse);
