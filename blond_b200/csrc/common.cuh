@@ -129,6 +129,12 @@ static __constant__ double kCos[9] = {
     -0.5,
 };
 
+// (-1)^k s, with k's parity in the low bit of its shifted sum ks: the sign bit
+// by shift and xor.
+__device__ __forceinline__ double flip_odd(double s, double ks) {
+    return __hiloint2double(__double2hiint(s) ^ (__double2loint(ks) << 31), __double2loint(s));
+}
+
 // sin(x) of an RF phase argument.  The FP64 particle passes spend much of
 // their issue slots on this sine, so it is written for the arguments they
 // see (|x| up to ~1e3 rad): Cody-Waite reduction by pi (W. J. Cody and
@@ -167,8 +173,7 @@ __device__ __forceinline__ double rf_sin(double x) {
     p = fma(p, r2, kSin[10]);
     p = fma(p, r2, kSin[11]);
     p = fma(p, r2, kSin[12]);
-    double s = fma(r * r2, p, r);
-    return (__double2loint(ks) & 1) ? -s : s;
+    return flip_odd(fma(r * r2, p, r), ks);
 }
 
 // sin(x) and cos(x) with rf_sin's reduction: cos(x) = (-1)^k cos(r), cos r
@@ -203,9 +208,8 @@ __device__ __forceinline__ void rf_sincos(double x, double* sp, double* cp) {
     q = fma(q, r2, kCos[7]);
     q = fma(q, r2, kCos[8]);
     const double c = fma(r2, q, 1.0);
-    const bool odd = (__double2loint(ks) & 1) != 0;
-    *sp = odd ? -s : s;
-    *cp = odd ? -c : c;
+    *sp = flip_odd(s, ks);
+    *cp = flip_odd(c, ks);
 }
 
 // sin(x) as a float for the F32P64 kick: k = rint(x / pi) by the shifter
@@ -225,7 +229,7 @@ __device__ __forceinline__ float rf_sinf(double x) {
     p = fmaf(p, r2, 0.00833333283662796f);
     p = fmaf(p, r2, -0.1666666716337204f);
     const float s = fmaf(r * r2, p, r);
-    return (__double2loint(ks) & 1) ? -s : s;
+    return __int_as_float(__float_as_int(s) ^ (__double2loint(ks) << 31));
 }
 
 __device__ __forceinline__ double dev_sin(double x) { return rf_sin(x); }

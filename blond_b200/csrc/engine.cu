@@ -288,17 +288,23 @@ static auto packed_kernel() {
     return particle_kernel_stab<PREC, SOLVER, NST, TAB>;
 }
 
+// The packed pass's prefetch setting that means the register pipeline.
+constexpr int kPipeRing = 1;
+
 template <int PREC, int SOLVER>
 static int launch_stab(blond_engine* e, const ParticleArgs& a, cudaStream_t s, bool launch) {
     const bool shared = e->variant == 2;
-    const int ring = shared ? (e->ring ? 2 : 0) : (e->ring >= 4 ? 4 : (e->ring ? 2 : 0));
+    const bool pipe = !shared && e->ring == kPipeRing;
+    const int ring = shared ? (e->ring ? 2 : 0)
+                            : (e->ring >= 4 ? 4 : (e->ring && !pipe ? 2 : 0));
     const int smem = shared ? stab_smem<PREC>(e, ring) : packed_smem<PREC>(e, ring);
     if (smem < 0) {
         set_error(shared ? "engine: the shared-table pass does not apply to this engine"
                          : "engine: the packed-histogram pass does not fit this engine");
         return BLOND_ERR_UNSUPPORTED;
     }
-    auto k = shared ? (ring ? packed_kernel<PREC, SOLVER, TAB_SHARED, 2>()
+    auto k = pipe ? particle_kernel_pipe<PREC, SOLVER>
+             : shared ? (ring ? packed_kernel<PREC, SOLVER, TAB_SHARED, 2>()
                             : packed_kernel<PREC, SOLVER, TAB_SHARED, 0>())
                     : (ring == 4 ? packed_kernel<PREC, SOLVER, TAB_GLOBAL, 4>()
                        : ring ? packed_kernel<PREC, SOLVER, TAB_GLOBAL, 2>()
@@ -308,7 +314,7 @@ static int launch_stab(blond_engine* e, const ParticleArgs& a, cudaStream_t s, b
     if (launch) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(device_info().sm_count, 1, 1);
-        cfg.blockDim = dim3(kEngineThreads, 1, 1);
+        cfg.blockDim = dim3(pipe ? kPipeThreads : kEngineThreads, 1, 1);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
@@ -1330,15 +1336,16 @@ static int time_graph_turns(blond_engine* e, cudaStream_t s, int turns, int reps
 }
 
 // Programmatic dependent launch on or off, whichever replays whole turns
-// faster with the chosen particle pass (the early launch of the next
-// kernel pays at short profiles and costs at long ones).  Each setting
+// faster with the particle pass that is set (the early launch of the next
+// kernel pays at short profiles and costs at long ones); turn_ms receives that
+// turn, or stays when nothing was timed.  Each setting
 // starts from the same snapshot of the turn counter, induced voltage and
 // profile, which are put back afterwards; the caller restores the beam and
 // histogram.  Skipped (overlap left as it is) with a beam-phase loop or
 // smooth slicing, whose turn state is not snapshotted, and when fewer
 // turns than it needs are left in the programme.
 static int tune_overlap(blond_engine* e, cudaStream_t s, const void* sdt, const void* sdE,
-                        const int* shist, int* chosen) {
+                        const int* shist, int* chosen, double* turn_ms) {
     constexpr int kTurns = 4, kReps = 3;
     *chosen = e->pdl ? 1 : 0;
     if (e->has_fb || e->smooth || e->host_turn + kTurns * (kReps + 1) > e->n_turns)
@@ -1380,6 +1387,7 @@ static int tune_overlap(blond_engine* e, cudaStream_t s, const void* sdt, const 
     // overlap stays on unless it is clearly slower
     e->pdl = rc == BLOND_OK ? !(t[0] < 0.97 * t[1]) : keep;
     *chosen = e->pdl ? 1 : 0;
+    if (rc == BLOND_OK) *turn_ms = t[*chosen];
     return rc;
 }
 
@@ -1455,8 +1463,10 @@ int blond_engine_autotune(blond_engine* e, int reps, void* stream, int* config,
     }
     // the plain pass with a packed histogram over the global table (long profiles)
     if (e->has_fft || e->has_ind || e->interp)
-        for (int ring : {0, 2, 4}) {
-            const int sm = f64 ? packed_smem<PREC_F64>(e, ring) : packed_smem<PREC_F32P64>(e, ring);
+        for (int ring : {0, kPipeRing, 2, 4}) {
+            const int stages = ring == kPipeRing ? 0 : ring;
+            const int sm = f64 ? packed_smem<PREC_F64>(e, stages)
+                               : packed_smem<PREC_F32P64>(e, stages);
             if (sm >= 0) cands.push_back({3, kEngineThreads, 1, HIST_PACKED, ring, 1, 0});
         }
     const Cand old = {e->variant, e->threads, e->blocks_per_sm, e->hist_mode, e->ring,
@@ -1466,6 +1476,8 @@ int blond_engine_autotune(blond_engine* e, int reps, void* stream, int* config,
     cudaEventCreate(&b);
     double best = 1e30;
     Cand win = old;
+    double best_of[4] = {1e30, 1e30, 1e30, 1e30};  // per kind of pass
+    Cand win_of[4] = {old, old, old, old};
     for (const Cand& c : cands) {
         e->variant = c.variant;
         e->hist_mode = c.hist;
@@ -1492,28 +1504,57 @@ int blond_engine_autotune(blond_engine* e, int reps, void* stream, int* config,
         }
         float ms = 0.f;
         cudaEventElapsedTime(&ms, a, b);
-        if (ms / reps < best) {
-            best = ms / reps;
-            win = c;
+        if (ms / reps < best_of[c.variant]) {
+            best_of[c.variant] = ms / reps;
+            win_of[c.variant] = c;
             if (c.variant == 0) {
-                win.threads = old.threads;
-                win.bps = old.bps;
+                win_of[0].threads = old.threads;
+                win_of[0].bps = old.bps;
             }
         }
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
-    // whole turns with the winner: overlap on or off
-    int overlap = e->pdl ? 1 : 0;
+    for (int v = 0; v < 4; ++v)
+        if (best_of[v] < best) {
+            best = best_of[v];
+            win = win_of[v];
+        }
+    // whole turns: every kind of pass within 20 % of the fastest, overlap on
+    // or off -- what a pass asks of the head and how much of it the pass
+    // overlaps count as well (Q32P64, 1e7 particles, 16384 slices: the packed
+    // pass is the faster one alone, but its turn takes 70 us, the shared-table
+    // pass's 65)
+    auto apply = [&](const Cand& c) {
+        e->variant = c.variant;
+        e->threads = c.threads;
+        e->blocks_per_sm = c.bps;
+        e->hist_mode = c.hist;
+        e->ring = c.ring;
+        e->cluster = c.cluster;
+        e->l2_ahead = c.l2 != 0;
+    };
+    const bool pdl0 = e->pdl;
+    int overlap = pdl0 ? 1 : 0;
     if (rc == BLOND_OK && best < 1e30) {
-        e->variant = win.variant;
-        e->threads = win.threads;
-        e->blocks_per_sm = win.bps;
-        e->hist_mode = win.hist;
-        e->ring = win.ring;
-        e->cluster = win.cluster;
-        e->l2_ahead = win.l2 != 0;
-        rc = tune_overlap(e, s, sdt, sdE, static_cast<const int*>(shist), &overlap);
+        const double fastest = best;
+        double best_turn = 1e30;
+        for (int v = 0; v < 4 && rc == BLOND_OK; ++v) {
+            if (best_of[v] > 1.2 * fastest) continue;
+            apply(win_of[v]);
+            e->pdl = pdl0;
+            int on = overlap;
+            double turn = 1e30;
+            rc = tune_overlap(e, s, sdt, sdE, static_cast<const int*>(shist), &on, &turn);
+            if (turn < best_turn) {
+                best_turn = turn;
+                best = best_of[v];
+                win = win_of[v];
+                overlap = on;
+            }
+        }
+        apply(win);
+        e->pdl = overlap != 0;
     }
     // restore the state of the run
     cudaMemcpyAsync(e->dt, sdt, 8 * n, cudaMemcpyDeviceToDevice, s);

@@ -99,14 +99,21 @@ __device__ __forceinline__ double energy_value(typename Coord<PREC>::E e, const 
 
 // Q32P64: counts + this turn's float64 energy increment, rounded once to
 // the grid.  A result beyond +-(2^31 - 1) counts (or a NaN increment) sets
-// the error word and saturates.
-__device__ __forceinline__ int q32_add(int q, double inc, const ParticleArgs& a) {
-    long long r = (long long)q + __double2ll_rn(__dmul_rn(inc, a.inv_lsb));
-    if (r > 2147483647LL || r < -2147483647LL) {
+// the error word and saturates.  `value` receives the new count as a double
+// (the drift needs it).  All in doubles: the rounding by the 1.5 * 2^52
+// shifter, whose low word then is the count -- a 64-bit integer conversion,
+// sum and two compares took eight instructions more.
+__device__ __forceinline__ int q32_add(int q, double inc, const ParticleArgs& a, double& value) {
+    const double shifter = kSin[0];
+    const double d = __dmul_rn(inc, a.inv_lsb);
+    const double k = __dsub_rn(__dadd_rn(d, shifter), shifter);  // rint for |d| < 2^51
+    double r = __dadd_rn((double)q, k);
+    if (!(fabs(r) <= 2147483647.0)) {
         if (a.err) atomicOr(a.err, ERR_ENERGY_RANGE);
-        r = r > 0 ? 2147483647LL : -2147483647LL;
+        r = r > 0.0 ? 2147483647.0 : -2147483647.0;
     }
-    return (int)r;
+    value = r;
+    return __double2loint(__dadd_rn(r, shifter));
 }
 
 // Table sources of the induced kick: the global table the head wrote, or a
@@ -175,7 +182,8 @@ __device__ __forceinline__ void track_one(double& t,
             }
             double s = 0.0;
             for (int j = 0; j < a.n_rf; ++j) s += c.V[j] * rf_sin(c.op[j].x * t + c.op[j].y);
-            e = q32_add(e, inc + (a.charge * s + c.acc), a);
+            double count;
+            e = q32_add(e, inc + (a.charge * s + c.acc), a, count);
         } else {
             if (LIK) {
                 const double f = floor((t - a.bc0) * a.lik_inv_w);
@@ -239,48 +247,60 @@ __device__ __forceinline__ void rf_sum_pair(const TurnConsts& c, int n_rf, doubl
     }
 }
 
+// The interpolation-table entries of two particles: gathered, in range or not,
+// and for F32P64 the offsets from the slice centres.
+template <int PREC>
+struct PairTable {
+    bool in0 = false, in1 = false;
+    typename TableEntry<PREC>::T tb0, tb1;
+    float x0f = 0.0f, x1f = 0.0f;
+};
+
+template <int PREC, int TAB>
+__device__ __forceinline__ void lookup_pair(double t0, double t1, const ParticleArgs& a,
+                                            const void* stab, PairTable<PREC>& p) {
+    // floor(y) in [0, S - 2] exactly when y is in [0, S - 1); the
+    // round-down conversion saturates outside the int range, so one
+    // unsigned compare tests it.  (A NaN y converts to 0 and takes
+    // entry 0; its particle's energy is NaN from the RF kick anyway.)
+    const double y0 = (t0 - a.bc0) * a.lik_inv_w;
+    const double y1 = (t1 - a.bc0) * a.lik_inv_w;
+    const int r0 = __double2int_rd(y0), r1 = __double2int_rd(y1);
+    p.in0 = (unsigned)r0 < (unsigned)(a.S - 1);
+    p.in1 = (unsigned)r1 < (unsigned)(a.S - 1);
+    const int k0 = p.in0 ? r0 : 0, k1 = p.in1 ? r1 : 0;
+    p.tb0 = table_at<PREC, TAB>(a, stab, k0);
+    p.tb1 = table_at<PREC, TAB>(a, stab, k1);
+    if (PREC == PREC_F32P64) {
+        // offsets from the slice centre, needed before t changes
+        p.x0f = (float)(t0 - (a.bc0 + (double)k0 * a.bw));
+        p.x1f = (float)(t1 - (a.bc0 + (double)k1 * a.bw));
+    }
+}
+
 // Two particles at once, with the interpolation-table gathers (L2-resident,
 // the longest-latency loads of the pass) issued before the RF sines so their
 // latency overlaps the sine arithmetic.  Same operations, in the same order
 // per particle, as two calls of track_one.
-template <int PREC, int SOLVER, bool LIK, int TAB = TAB_GLOBAL, bool RF2 = false>
-__device__ __forceinline__ void track_pair(double& t0, double& t1,
-                                           typename Coord<PREC>::E& e0,
-                                           typename Coord<PREC>::E& e1,
-                                           const TurnConsts& c, const ParticleArgs& a,
-                                           int order, const void* stab = nullptr) {
+template <int PREC, int SOLVER, bool LIK, bool RF2 = false>
+__device__ __forceinline__ void track_pair_with(double& t0, double& t1,
+                                                typename Coord<PREC>::E& e0,
+                                                typename Coord<PREC>::E& e1,
+                                                const TurnConsts& c, const ParticleArgs& a,
+                                                int order, const PairTable<PREC>& p) {
     using E = typename Coord<PREC>::E;
-    using TB = typename TableEntry<PREC>::T;
-    bool in0 = false, in1 = false;
-    TB tb0, tb1;
-    float x0f = 0.0f, x1f = 0.0f;  // F32P64: offsets from the slice centre
-    if (LIK) {
-        // floor(y) in [0, S - 2] exactly when y is in [0, S - 1); the
-        // round-down conversion saturates outside the int range, so one
-        // unsigned compare tests it.  (A NaN y converts to 0 and takes
-        // entry 0; its particle's energy is NaN from the RF kick anyway.)
-        const double y0 = (t0 - a.bc0) * a.lik_inv_w;
-        const double y1 = (t1 - a.bc0) * a.lik_inv_w;
-        const int r0 = __double2int_rd(y0), r1 = __double2int_rd(y1);
-        in0 = (unsigned)r0 < (unsigned)(a.S - 1);
-        in1 = (unsigned)r1 < (unsigned)(a.S - 1);
-        const int k0 = in0 ? r0 : 0, k1 = in1 ? r1 : 0;
-        tb0 = table_at<PREC, TAB>(a, stab, k0);
-        tb1 = table_at<PREC, TAB>(a, stab, k1);
-        if (PREC == PREC_F32P64) {
-            // offsets from the slice centre, needed before t changes
-            x0f = (float)(t0 - (a.bc0 + (double)k0 * a.bw));
-            x1f = (float)(t1 - (a.bc0 + (double)k1 * a.bw));
-        }
-    }
+    double d0, d1;  // the new energies in eV
     if constexpr (PREC == PREC_Q32P64) {
         // the turn's whole energy change in float64, rounded once per particle
         double x0 = 0.0, x1 = 0.0;
         rf_sum_pair<RF2>(c, a.n_rf, t0, t1, x0, x1);
-        const double i0 = (LIK && in0) ? __fma_rn(t0, tb0.x, tb0.y) : 0.0;
-        const double i1 = (LIK && in1) ? __fma_rn(t1, tb1.x, tb1.y) : 0.0;
-        e0 = q32_add(e0, i0 + (a.charge * x0 + c.acc), a);
-        e1 = q32_add(e1, i1 + (a.charge * x1 + c.acc), a);
+        const double i0 = (LIK && p.in0) ? __fma_rn(t0, p.tb0.x, p.tb0.y) : 0.0;
+        const double i1 = (LIK && p.in1) ? __fma_rn(t1, p.tb1.x, p.tb1.y) : 0.0;
+        double n0, n1;
+        e0 = q32_add(e0, i0 + (a.charge * x0 + c.acc), a, n0);
+        e1 = q32_add(e1, i1 + (a.charge * x1 + c.acc), a, n1);
+        d0 = __dmul_rn(n0, a.lsb);  // energy_value
+        d1 = __dmul_rn(n1, a.lsb);
     } else {
         E s0, s1;
         if (PREC == PREC_F64) {
@@ -313,18 +333,21 @@ __device__ __forceinline__ void track_pair(double& t0, double& t1,
         }
         if (LIK) {
             if (PREC == PREC_F64) {
-                if (in0) e0 = __dadd_rn(e0, __fma_rn(t0, tb0.x, tb0.y));
-                if (in1) e1 = __dadd_rn(e1, __fma_rn(t1, tb1.x, tb1.y));
+                if (p.in0) e0 = __dadd_rn(e0, __fma_rn(t0, p.tb0.x, p.tb0.y));
+                if (p.in1) e1 = __dadd_rn(e1, __fma_rn(t1, p.tb1.x, p.tb1.y));
             } else {
-                if (in0) e0 += __fmaf_rn(tb0.y, x0f, tb0.x);
-                if (in1) e1 += __fmaf_rn(tb1.y, x1f, tb1.x);
+                if (p.in0) e0 += __fmaf_rn(p.tb0.y, p.x0f, p.tb0.x);
+                if (p.in1) e1 += __fmaf_rn(p.tb1.y, p.x1f, p.tb1.x);
             }
         }
         const E q = (E)a.charge, acc = (E)c.acc;
         e0 += q * s0 + acc;
         e1 += q * s1 + acc;
     }
-    const double d0 = energy_value<PREC>(e0, a), d1 = energy_value<PREC>(e1, a);
+    if constexpr (PREC != PREC_Q32P64) {
+        d0 = (double)e0;
+        d1 = (double)e1;
+    }
     if (SOLVER == BLOND_SOLVER_SIMPLE) {
         t0 = drift_simple<double>(t0, d0, c.d.simple);
         t1 = drift_simple<double>(t1, d1, c.d.simple);
@@ -337,6 +360,17 @@ __device__ __forceinline__ void track_pair(double& t0, double& t1,
         t1 = drift_exact<double>(t1, d1, c.d.Tr, c.d.ib2, c.d.ie2, c.d.a0, c.d.a1,
                                  c.d.a2, c.d.energy);
     }
+}
+
+template <int PREC, int SOLVER, bool LIK, int TAB = TAB_GLOBAL, bool RF2 = false>
+__device__ __forceinline__ void track_pair(double& t0, double& t1,
+                                           typename Coord<PREC>::E& e0,
+                                           typename Coord<PREC>::E& e1,
+                                           const TurnConsts& c, const ParticleArgs& a,
+                                           int order, const void* stab = nullptr) {
+    PairTable<PREC> p;
+    if constexpr (LIK) lookup_pair<PREC, TAB>(t0, t1, a, stab, p);
+    track_pair_with<PREC, SOLVER, LIK, RF2>(t0, t1, e0, e1, c, a, order, p);
 }
 
 __device__ __forceinline__ int engine_bin(double t, double cut_left, double inv_w, int S) {
@@ -935,6 +969,96 @@ particle_kernel_stab(const ParticleArgs a) {
         dt[a.n - 1] = t;
         dE[a.n - 1] = e;
         deposit_packed(sh, half, a.hist, engine_bin(t, a.cut_left, a.inv_w, S));
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < half; k += blockDim.x) {
+        const unsigned v = sh[k];
+        if (v & 0xffffu) atomicAdd(&a.hist[k], (int)(v & 0xffffu));
+        if ((v >> 16) && k + half < S) atomicAdd(&a.hist[k + half], (int)(v >> 16));
+    }
+}
+
+// The packed pass with its loads in a register pipeline: while a thread
+// computes one pair, the table entries of its next pair and the coordinates of
+// the one after are on their way.  Long profiles gather from L2 (1 MB at 2^16
+// slices) and leave no shared memory for a ring, so the pass above waits for
+// both one after the other (ncu: 4.5 long-scoreboard stalls per issue, issue
+// active 61 %).  768 threads: 80 registers.
+constexpr int kPipeThreads = 768;
+
+template <int PREC, int SOLVER>
+__global__ void __launch_bounds__(kPipeThreads, 1)
+particle_kernel_pipe(const ParticleArgs a) {
+    using E = typename Coord<PREC>::E;
+    using E2 = typename Vec2<E>::type;
+    extern __shared__ __align__(16) unsigned char psm[];
+    __shared__ TurnConsts c;
+    pdl_launch_dependents();
+    const int S = a.S, half = (S + 1) / 2;
+    unsigned* const sh = reinterpret_cast<unsigned*>(psm);
+    for (int k = threadIdx.x; k < half; k += blockDim.x) sh[k] = 0u;
+    pdl_wait();  // the head's table, counter and cleared histogram
+    long long t_idx = a.turn ? (*a.turn - 1) : 0;
+    if (t_idx < 0) t_idx = 0;
+    if (t_idx >= a.n_turns) t_idx = a.n_turns - 1;
+    for (int j = threadIdx.x; j < a.n_rf; j += blockDim.x) {
+        c.V[j] = a.V[t_idx * a.n_rf + j];
+        c.Vf[j] = (float)c.V[j];
+        c.op[j] = make_double2(a.om[t_idx * a.n_rf + j], a.ph[t_idx * a.n_rf + j]);
+    }
+    if (threadIdx.x == 0) {
+        c.acc = a.interp ? 0.0 : a.acc[t_idx];
+        c.d = a.drift[t_idx + 1];
+    }
+    double2* const dt = reinterpret_cast<double2*>(a.dt);
+    E2* const dE = reinterpret_cast<E2*>(a.dE);
+    const int64_t npairs = a.n / 2;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const uint64_t pol = evict_first_policy();
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double2 t, tn;
+    E2 e, en;
+    if (i < npairs) {
+        t = stream_load(dt + i, pol);
+        e = stream_load(dE + i, pol);
+    }
+    if (i + stride < npairs) {
+        tn = stream_load(dt + i + stride, pol);
+        en = stream_load(dE + i + stride, pol);
+    }
+    PairTable<PREC> p;
+    if (i < npairs) lookup_pair<PREC, TAB_GLOBAL>(t.x, t.y, a, nullptr, p);
+    __syncthreads();
+    for (; i < npairs; i += stride) {
+        PairTable<PREC> pn;
+        double2 t2;
+        E2 e2;
+        if (i + stride < npairs) lookup_pair<PREC, TAB_GLOBAL>(tn.x, tn.y, a, nullptr, pn);
+        if (i + 2 * stride < npairs) {
+            t2 = stream_load(dt + i + 2 * stride, pol);
+            e2 = stream_load(dE + i + 2 * stride, pol);
+        }
+        track_pair_with<PREC, SOLVER, true>(t.x, t.y, e.x, e.y, c, a, a.order, p);
+        stream_store(dt + i, t, pol);
+        stream_store(dE + i, e, pol);
+        deposit_packed(sh, half, a.hist, engine_bin(t.x, a.cut_left, a.inv_w, S));
+        deposit_packed(sh, half, a.hist, engine_bin(t.y, a.cut_left, a.inv_w, S));
+        t = tn;
+        e = en;
+        tn = t2;
+        en = e2;
+        p = pn;
+    }
+    // odd tail particle
+    if ((a.n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        double* const d = reinterpret_cast<double*>(a.dt) + a.n - 1;
+        E* const q = reinterpret_cast<E*>(a.dE) + a.n - 1;
+        double x = *d;
+        E y = *q;
+        track_one<PREC, SOLVER, true, true, true, false, TAB_GLOBAL>(x, y, c, a, nullptr, a.order);
+        *d = x;
+        *q = y;
+        deposit_packed(sh, half, a.hist, engine_bin(x, a.cut_left, a.inv_w, S));
     }
     __syncthreads();
     for (int k = threadIdx.x; k < half; k += blockDim.x) {
