@@ -17,6 +17,7 @@
 // captured once and replayed.
 #include "engine_device.cuh"
 #include "convolve.cuh"
+#include "head_fft.cuh"
 
 using namespace bb;
 
@@ -1050,13 +1051,6 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
                   "profile (%d slices)", (long long)n_fft, e->S);
     int rc = upload((void**)&e->d_H, Z, sizeof(double2) * (size_t)(n_fft / 2 + 1));
     if (rc) return rc;
-    // twiddle tables of this plan, computed once instead of every turn
-    free_ptr(e->d_tw);
-    e->d_tw = nullptr;
-    if ((rc = make_spec_twiddles(plan, &e->d_tw))) return rc;
-    e->plan = plan;
-    e->iv_scale = scale;
-    e->has_fft = true;
     // short profiles: the direct convolution's impulse response
     e->conv = false;
     free_ptr(e->d_hx);
@@ -1069,7 +1063,22 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
         if ((rc = make_conv_response(e->d_H, n_fft, e->S, 1, &e->d_hx))) return rc;
         if ((rc = prepare_conv())) return rc;
         e->conv = true;
+    } else if (const int64_t P = head_fft_length(n_fft, e->S)) {
+        // long profiles at other lengths: the same voltages by the
+        // power-of-two transform
+        double2* H = nullptr;
+        if ((rc = make_head_response(e->d_H, n_fft, e->S, P, &H))) return rc;
+        free_ptr(e->d_H);
+        e->d_H = H;
+        make_spec_plan(P, plan);
     }
+    // twiddle tables of this plan, computed once instead of every turn
+    free_ptr(e->d_tw);
+    e->d_tw = nullptr;
+    if ((rc = make_spec_twiddles(plan, &e->d_tw))) return rc;
+    e->plan = plan;
+    e->iv_scale = scale;
+    e->has_fft = true;
     e->graph_dirty = true;
     return BLOND_OK;
 }

@@ -100,10 +100,11 @@ struct HeadShape {
     // the two-level tables' split, as make_spec_plan chooses it
     static constexpr int lgL = (lgM1 + lgM2 + 1) / 2, L = 1 << lgL, nA = (M + L - 1) / L;
     static constexpr int tw_count = M1 + M2 + 2 * nA + 2 * L;
-    // bytes: columns, rows, twiddles, impedance, voltages and their neighbours
+    // bytes: columns, rows (at the end the voltages), twiddles, impedance and
+    // the neighbour's voltages
     static constexpr int o_rows = 16 * Bc * ldc, o_tw = o_rows + 16 * Br * ldr,
-                         o_h = o_tw + 16 * tw_count, o_v = o_h + 16 * (per + 1),
-                         o_nbr = o_v + 16 * per, bytes = o_nbr + 8 * M1;
+                         o_h = o_tw + 16 * tw_count, o_nbr = o_h + 16 * (per + 1),
+                         bytes = o_nbr + 8 * M1;
     static_assert(Br >= 2 && Bc >= 1, "16 CTAs");
 };
 
@@ -142,7 +143,7 @@ head_fft_kernel(const SpecParams P) {
     double2* const tan_ = tbm + Sh::L;
     double2* const tbn = tan_ + Sh::nA;
     double2* const hk = reinterpret_cast<double2*>(hsm + Sh::o_h);
-    double2* const vloc = reinterpret_cast<double2*>(hsm + Sh::o_v);
+    double2* const vloc = rows;  // per <= Br (M2 + 1) values, free by then
     double* const nbr = reinterpret_cast<double*>(hsm + Sh::o_nbr);
     // every CTA of the cluster runs (its shared memory may be written) once
     // this barrier, waited for before the first push, has completed
@@ -363,6 +364,7 @@ bool for_shape(int M1, int M2, F f) {
     else if (M1 == 64 && M2 == 128) f(head_fft_kernel<2, 4>, HeadShape<2, 4>{});
     else if (M1 == 128 && M2 == 128) f(head_fft_kernel<4, 4>, HeadShape<4, 4>{});
     else if (M1 == 128 && M2 == 256) f(head_fft_kernel<4, 8>, HeadShape<4, 8>{});
+    else if (M1 == 256 && M2 == 256) f(head_fft_kernel<8, 8>, HeadShape<8, 8>{});
     else return false;
     return true;
 }
@@ -380,14 +382,62 @@ bool head_fft_takes(const SpecParams& P) {
            fits;
 }
 
+// h_{d mod N} for |d| < S at position d mod M (the rest 0).
+__global__ void extend_response_kernel(const double* y, int64_t N, int S, int64_t P, double* h) {
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < P;
+         x += (int64_t)gridDim.x * blockDim.x)
+        h[x] = x < S ? y[x] : (x > P - S ? y[N - (P - x)] : 0.0);
+}
+
+int64_t head_fft_length(int64_t N, int S) {
+    if ((N & (N - 1)) == 0 || N < S) return 0;
+    int64_t P = 8192;
+    while (P < 2 * (int64_t)S - 1) P *= 2;
+    SpecPlan plan;
+    if (P > kMaxClusterFFT || !make_spec_plan(P, plan)) return 0;
+    SpecParams q = {};
+    q.p = plan;
+    q.mode = SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE;
+    q.n_in = q.n_out = S;
+    return head_fft_takes(q) ? P : 0;
+}
+
+int make_head_response(const double2* H, int64_t N, int S, int64_t P, double2** out) {
+    *out = nullptr;
+    double* y = nullptr;
+    BB_CUDA(cudaMalloc((void**)&y, sizeof(double) * (size_t)(N + P)));
+    int rc = blond_irfft_f64(reinterpret_cast<const double*>(H), N, y, N, nullptr);
+    if (rc == BLOND_OK) {
+        extend_response_kernel<<<64, 256>>>(y, N, S, P, y + N);
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMalloc((void**)out, sizeof(double2) * (size_t)(P / 2 + 1)) != cudaSuccess) {
+            set_error("head: building the response failed");
+            rc = BLOND_ERR_CUDA;
+        }
+    }
+    if (rc == BLOND_OK)
+        rc = blond_rfft_f64(y + N, P, P, reinterpret_cast<double*>(*out), nullptr);
+    if (rc == BLOND_OK && cudaDeviceSynchronize() != cudaSuccess) {
+        set_error("head: building the response failed");
+        rc = BLOND_ERR_CUDA;
+    }
+    cudaFree(y);
+    if (rc && *out) {
+        cudaFree(*out);
+        *out = nullptr;
+    }
+    return rc;
+}
+
 int prepare_head_fft() {
     static bool done[64] = {false};
     const DeviceInfo& d = device_info();
     if (done[d.device & 63]) return BLOND_OK;
     cudaError_t rc = cudaSuccess;
-    const int shapes[4][2] = {{64, 64}, {64, 128}, {128, 128}, {128, 256}};
+    const int shapes[5][2] = {{64, 64}, {64, 128}, {128, 128}, {128, 256}, {256, 256}};
     for (const auto& s : shapes)
         for_shape(s[0], s[1], [&](auto k, auto sh) {
+            if (sh.bytes > d.max_smem_optin) return;
             if (rc == cudaSuccess)
                 rc = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (rc == cudaSuccess)
