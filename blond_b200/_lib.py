@@ -10,6 +10,8 @@ import ctypes as ct
 import os
 import threading
 
+import torch
+
 from .build import LIB
 
 _lock = threading.Lock()
@@ -188,10 +190,28 @@ def load(path: str | None = None) -> ct.CDLL:
         return lib
 
 
+_functions = {}  # name -> bound entry point of the loaded library
+
+
 def call(name: str, *args) -> None:
     """Call an entry point and raise BlondB200Error on a non-zero status."""
-    lib = load()
-    rc = getattr(lib, name)(*args)
+    fn = _functions.get(name)
+    if fn is None:
+        fn = _functions[name] = getattr(load(), name)
+    rc = fn(*args)
     if rc != OK:
-        msg = lib.blond_b200_last_error().decode(errors="replace")
+        msg = load().blond_b200_last_error().decode(errors="replace")
         raise BlondB200Error(name, rc, msg)
+
+
+def stream() -> int:
+    """The current stream of torch's current device, as its raw handle (a
+    torch.cuda.Stream object costs 3 us to make, a small call's launch 3)."""
+    return _raw_stream(torch.cuda.current_device())
+
+
+def _raw_stream_from_object(device: int) -> int:
+    return torch.cuda.current_stream(device).cuda_stream
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _raw_stream_from_object)

@@ -43,8 +43,7 @@ def _p(t: torch.Tensor | None) -> ct.c_void_p:
     return ct.c_void_p(t.data_ptr() if t is not None else 0)
 
 
-def _stream() -> ct.c_void_p:
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.stream
 
 
 def resonator_impedance(R_S, frequency_R, Q, n_fft: int, bin_size: float) -> torch.Tensor:

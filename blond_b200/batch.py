@@ -31,8 +31,7 @@ def _p(a: np.ndarray) -> ct.c_void_p:
     return a.ctypes.data_as(ct.c_void_p)
 
 
-def _stream():
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.stream
 
 
 class BatchTracker:

@@ -54,12 +54,11 @@ def use_precision(p: str = "double") -> None:
     precision.set(p)
 
 
-def _stream() -> ct.c_void_p:
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.stream
 
 
-def _ptr(t: torch.Tensor) -> ct.c_void_p:
-    return ct.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()
 
 
 def _suffix(t: torch.Tensor) -> str:
@@ -85,6 +84,10 @@ def _check_particles(*arrays: torch.Tensor) -> None:
 
 def as_device(x, dtype: torch.dtype, device=None) -> torch.Tensor:
     """Small parameter array -> contiguous CUDA tensor of ``dtype``."""
+    if isinstance(x, torch.Tensor) and x.dtype == dtype and x.is_cuda and x.is_contiguous() \
+            and (x.device == device if device is not None
+                 else x.get_device() == torch.cuda.current_device()):
+        return x
     if device is None:
         device = torch.device("cuda", torch.cuda.current_device())
     if isinstance(x, torch.Tensor):
@@ -101,13 +104,17 @@ def _real(t: torch.Tensor):
 def kick(dt, dE, voltage, omega_rf, phi_rf, charge, n_rf, acceleration_kick):
     """butils_wrap_cpp.kick (:863-898) -> cpp_routines/kick.cpp:16-35."""
     _check_particles(dt, dE)
-    r = _real(dt)
     V = as_device(voltage, dt.dtype, dt.device)
     om = as_device(omega_rf, dt.dtype, dt.device)
     ph = as_device(phi_rf, dt.dtype, dt.device)
-    _lib.call(f"blond_kick_{_suffix(dt)}", _ptr(dt), _ptr(dE), int(n_rf),
-              r(float(charge)), _ptr(V), _ptr(om), _ptr(ph), dt.numel(),
-              r(float(acceleration_kick)), _stream())
+    _kick(dt, dE, V.data_ptr(), om.data_ptr(), ph.data_ptr(), charge, n_rf, acceleration_kick)
+
+
+def _kick(dt, dE, V, om, ph, charge, n_rf, acceleration_kick):
+    """kick() with checked particle arrays and the addresses of RF arrays of
+    their type."""
+    _lib.call(f"blond_kick_{_suffix(dt)}", dt.data_ptr(), dE.data_ptr(), int(n_rf),
+              float(charge), V, om, ph, dt.numel(), float(acceleration_kick), _stream())
 
 
 def rf_volt_comp(voltages, omega_rf, phi_rf, bin_centers):
@@ -131,31 +138,25 @@ def drift(dt, dE, solver, t_rev, length_ratio, alpha_order, eta_0, eta_1,
     _check_particles(dt, dE)
     if solver not in _SOLVERS:
         raise KeyError(solver)
-    r = _real(dt)
-    vals = [t_rev, length_ratio, alpha_order, eta_0, eta_1, eta_2, alpha_0,
-            alpha_1, alpha_2, beta, energy]
-    _lib.call(f"blond_drift_{_suffix(dt)}", _ptr(dt), _ptr(dE),
-              _SOLVERS[solver], *[r(float(v)) for v in vals], dt.numel(),
-              _stream())
+    _lib.call(f"blond_drift_{_suffix(dt)}", _ptr(dt), _ptr(dE), _SOLVERS[solver],
+              float(t_rev), float(length_ratio), float(alpha_order), float(eta_0),
+              float(eta_1), float(eta_2), float(alpha_0), float(alpha_1), float(alpha_2),
+              float(beta), float(energy), dt.numel(), _stream())
 
 
 # ------------------------------------------------------------------ slicing
 def slice_beam(dt, profile, cut_left, cut_right):
     """butils_wrap_cpp.slice_beam (:971-984) -> histogram.cpp:22-73."""
     _check_particles(dt, profile)
-    r = _real(dt)
     _lib.call(f"blond_histogram_{_suffix(dt)}", _ptr(dt), _ptr(profile),
-              r(float(cut_left)), r(float(cut_right)), profile.numel(),
-              dt.numel(), _stream())
+              float(cut_left), float(cut_right), profile.numel(), dt.numel(), _stream())
 
 
 def slice_smooth(dt, profile, cut_left, cut_right):
     """butils_wrap_cpp.slice_smooth (:987-999) -> histogram.cpp:75-132."""
     _check_particles(dt, profile)
-    r = _real(dt)
     _lib.call(f"blond_smooth_histogram_{_suffix(dt)}", _ptr(dt), _ptr(profile),
-              r(float(cut_left)), r(float(cut_right)), profile.numel(),
-              dt.numel(), _stream())
+              float(cut_left), float(cut_right), profile.numel(), dt.numel(), _stream())
 
 
 # ------------------------------------------------------ interpolated kick
@@ -163,12 +164,11 @@ def linear_interp_kick(dt, dE, voltage, bin_centers, charge,
                        acceleration_kick):
     """butils_wrap_cpp.linear_interp_kick (:946-968)."""
     _check_particles(dt, dE)
-    r = _real(dt)
     V = as_device(voltage, dt.dtype, dt.device)
     bc = as_device(bin_centers, dt.dtype, dt.device)
     _lib.call(f"blond_linear_interp_kick_{_suffix(dt)}", _ptr(dt), _ptr(dE),
-              _ptr(V), _ptr(bc), r(float(charge)), bc.numel(), dt.numel(),
-              r(float(acceleration_kick)), _stream())
+              _ptr(V), _ptr(bc), float(charge), bc.numel(), dt.numel(),
+              float(acceleration_kick), _stream())
 
 
 # ------------------------------------------------------- impedance / FFT
@@ -231,7 +231,8 @@ def induced_voltage_1turn(profile, total_impedance, n_fft, scale, n_out):
     Z = total_impedance if isinstance(total_impedance, torch.Tensor) else \
         torch.as_tensor(np.asarray(total_impedance, np.complex128),
                         device=p.device)
-    Z = Z.to(torch.complex128).contiguous()
+    if Z.dtype != torch.complex128 or not Z.is_contiguous():
+        Z = Z.to(torch.complex128).contiguous()
     out = torch.empty(int(n_out), dtype=torch.float64, device=p.device)
     _lib.call("blond_induced_voltage_f64", _ptr(p), p.numel(), _ptr(Z),
               int(n_fft), float(scale), _ptr(out), int(n_out), _stream())
@@ -371,12 +372,11 @@ def resonator_induced_voltage(profile, bin_centers, bin_size, beam_n_macropartic
     forward by ``shift`` points (zeros behind) plus the voltage on its first
     n_time points (impedance.py:1317-1335), n_memory values.
     Returns (induced_voltage or memory, workspace)."""
-    p = as_device(profile, torch.float64).reshape(-1).contiguous()
-    bc = as_device(bin_centers, torch.float64, p.device).reshape(-1).contiguous()
-    t = as_device(time_array, torch.float64, p.device).reshape(-1).contiguous()
-    Rh = np.ascontiguousarray(np.asarray(R, dtype=np.float64).reshape(-1))
-    wh = np.ascontiguousarray(np.asarray(omega_r, dtype=np.float64).reshape(-1))
-    qh = np.ascontiguousarray(np.asarray(Q, dtype=np.float64).reshape(-1))
+    p = as_device(profile, torch.float64)
+    bc = as_device(bin_centers, torch.float64, p.device)
+    t = as_device(time_array, torch.float64, p.device)
+    Rh, wh, qh = (np.ascontiguousarray(x, dtype=np.float64).reshape(-1)
+                  for x in (R, omega_r, Q))
     n_res = Rh.size
     if not (wh.size == qh.size == n_res):
         raise ValueError("R, omega_r and Q differ in length")
@@ -384,7 +384,7 @@ def resonator_induced_voltage(profile, bin_centers, bin_size, beam_n_macropartic
         raise ValueError("profile and bin_centers differ in length")
     if workspace is None:
         workspace = resonator_workspace(bc.numel(), n_res, p.device)
-    P = lambda a: a.ctypes.data_as(ct.c_void_p)  # noqa: E731
+    P = lambda a: a.ctypes.data  # noqa: E731
     tm = _ptr(tmp_matrix) if tmp_matrix is not None else None
     if memory_in is not None:
         mem = memory_in

@@ -120,7 +120,9 @@ int stats_impl(const T* dt, const T* dE, const int64_t* id, int64_t n, double* s
                      aligned(scratch, 8) && aligned(ticket, 4) && (!id || aligned(id, 8)),
                  "beam_statistics: misaligned array");
     const DeviceInfo& d = device_info();
-    int64_t grid = (n + kStatThreads - 1) / kStatThreads;
+    // four elements a thread and iteration: fewer partials for the last block
+    // (3e5 particles 9.1 -> 7.4 us)
+    int64_t grid = (n + 4 * kStatThreads - 1) / (4 * kStatThreads);
     grid = grid < (int64_t)d.sm_count * 8 ? grid : (int64_t)d.sm_count * 8;
     if (grid > BLOND_STATS_MAX_BLOCKS) grid = BLOND_STATS_MAX_BLOCKS;
     stats_kernel<T><<<(int)grid, kStatThreads, 0, as_stream(stream)>>>(dt, dE, id, n, stats,

@@ -5,6 +5,7 @@
 #include "spectral.cuh"
 #include "head_fft.cuh"
 
+#include <mutex>
 #include <vector>
 
 namespace bb {
@@ -177,6 +178,50 @@ int make_spec_twiddles(const SpecPlan& plan, double2** out) {
     return BLOND_OK;
 }
 
+// Twiddle tables of the transforms called by themselves, made once per plan
+// and device and kept (at most kKeptTables of at most ~50 KB; further plans
+// compute theirs in the kernel, as does a call under capture whose table is
+// not there yet).  A table is complete before its address is handed out and is
+// never changed or freed, so calls of all threads and streams share it.
+constexpr int kKeptTables = 32;
+
+static const double2* shared_twiddles(const SpecPlan& plan, cudaStream_t stream) {
+    struct Kept {
+        int device, M1, M2;
+        double2* table;
+    };
+    static Kept kept[kKeptTables];
+    static int n_kept = 0;
+    static std::mutex mu;
+    const int dev = device_info().device;
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < n_kept; ++i)
+        if (kept[i].device == dev && kept[i].M1 == plan.M1 && kept[i].M2 == plan.M2)
+            return kept[i].table;
+    cudaStreamCaptureStatus cs;
+    if (n_kept == kKeptTables || cudaStreamIsCapturing(stream, &cs) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusNone)
+        return nullptr;
+    // another thread's capture is none of this allocation's business
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    double2* table = nullptr;
+    cudaStream_t own = nullptr;
+    bool ok = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaMalloc((void**)&table, spec_twiddle_bytes(plan)) == cudaSuccess &&
+              fill_spec_twiddles(plan, table, own) == BLOND_OK &&
+              cudaStreamSynchronize(own) == cudaSuccess;
+    if (own) cudaStreamDestroy(own);
+    if (!ok && table) cudaFree(table);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    kept[n_kept++] = {dev, plan.M1, plan.M2, table};
+    return table;
+}
+
 // ---------------------------------------------------------------- direct DFT
 // Single-CTA O(N^2) transforms for short lengths the cluster plan rejects.
 // Twiddles are indexed (k n mod N) from a shared table.
@@ -267,6 +312,7 @@ int blond_rfft_f64(const double* x, int64_t n_x, int64_t n_fft, double* spectrum
         P.in_f64 = x;
         P.n_in = n_x;
         P.spec_out = reinterpret_cast<double2*>(spectrum);
+        P.twg = shared_twiddles(P.p, s);
         return launch_spectral(P, s);
     }
     if (n_fft > kMaxDirectDFT) {
@@ -297,6 +343,7 @@ int blond_irfft_f64(const double* spectrum, int64_t n_fft, double* y,
         P.out = y;
         P.n_out = n_out;
         P.out_scale = 1.0 / (double)P.p.M;
+        P.twg = shared_twiddles(P.p, s);
         return launch_spectral(P, s);
     }
     if (n_fft > kMaxDirectDFT) {
@@ -330,6 +377,7 @@ int blond_induced_voltage_f64(const double* profile, int n_slices,
         P.out = v_out;
         P.n_out = n_out < n_fft ? n_out : n_fft;
         P.out_scale = -scale / (double)P.p.M;
+        P.twg = shared_twiddles(P.p, s);
         return launch_spectral(P, s);
     }
     set_error("induced_voltage: n_fft=%lld is not an even 5-smooth length <= %lld; "

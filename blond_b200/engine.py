@@ -98,8 +98,7 @@ class TurnEngine:
 FB_MACHINES = {"LHC": 1, "LHC_F": 2, "SPS_F": 3, "SPS_RL": 4, "PSB": 5}
 
 
-def _stream():
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.stream
 
 
 def start_sharded(slice_local, reduce, refresh):
@@ -377,7 +376,7 @@ class FusedTracker:
         """Advance n_turns; updates the RF counter and beam energy fields."""
         self._maybe_tune()
         if self.group is None:
-            self.eng.call("run", int(n_turns), _stream())
+            _lib.call("blond_engine_run", self.eng.h, int(n_turns), _stream())
         else:
             run_sharded_turns(n_turns, lambda: self.eng.call("step", 1, _stream()),
                               lambda: self.eng.call("step", 2, _stream()), self._reduce,
@@ -461,10 +460,10 @@ class FusedTracker:
 
     def profile_tensor(self) -> torch.Tensor:
         prof = torch.empty(self.profile.n_slices, dtype=torch.float64, device="cuda")
-        self.eng.call("get_profile", ct.c_void_p(prof.data_ptr()), _stream())
+        _lib.call("blond_engine_get_profile", self.eng.h, prof.data_ptr(), _stream())
         return prof
 
     def induced_voltage_tensor(self) -> torch.Tensor:
         v = torch.empty(self.profile.n_slices, dtype=torch.float64, device="cuda")
-        self.eng.call("get_induced_voltage", ct.c_void_p(v.data_ptr()), _stream())
+        _lib.call("blond_engine_get_induced_voltage", self.eng.h, v.data_ptr(), _stream())
         return v

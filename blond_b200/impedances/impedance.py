@@ -14,6 +14,7 @@ blond_resonator_induced_voltage_f64.
 """
 from __future__ import annotations
 
+import functools
 import warnings
 
 import numpy as np
@@ -47,6 +48,7 @@ def induced_voltage_lengths(n_slices: int, bin_size: float, cut_left: float,
                        "can be specified.")
 
 
+@functools.lru_cache(maxsize=256)
 def _smooth_even(n: int) -> bool:
     if n < 2 or n % 2:
         return False

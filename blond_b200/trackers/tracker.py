@@ -67,9 +67,16 @@ class RingAndRFTracker:
     def kick(self, beam_dt, beam_dE, index: int):
         """tracker.py:399-422."""
         V, om, ph = self._programme()
-        bm.kick(beam_dt, beam_dE, V[index], om[index], ph[index],
-                self.rf_params.particle.charge, self.rf_params.n_rf,
-                self.acceleration_kick[index])
+        if beam_dt.dtype != V.dtype or not 0 <= index < V.shape[0]:
+            return bm.kick(beam_dt, beam_dE, V[index], om[index], ph[index],
+                           self.rf_params.particle.charge, self.rf_params.n_rf,
+                           self.acceleration_kick[index])
+        # column `index` of the turn-major programmes, by address
+        bm._check_particles(beam_dt, beam_dE)
+        off = int(index) * V.stride(0) * V.element_size()
+        bm._kick(beam_dt, beam_dE, V.data_ptr() + off, om.data_ptr() + off, ph.data_ptr() + off,
+                 self.rf_params.particle.charge, self.rf_params.n_rf,
+                 self.acceleration_kick[index])
 
     def drift(self, beam_dt, beam_dE, index: int):
         """tracker.py:424-468."""
@@ -96,10 +103,15 @@ class RingAndRFTracker:
         if self.beamFB is not None and turn >= self.beamFB.delay:
             self.beamFB.track()
             self._sync_column(1, turn + 1)
-        rf.dphi_rf += (2.0 * np.pi * rf.harmonic[:, turn + 1]
-                       * (rf.omega_rf[:, turn + 1] - rf.omega_rf_d[:, turn + 1])
-                       / rf.omega_rf_d[:, turn + 1])
-        if np.any(rf.dphi_rf != 0):
+        # (element by element: numpy's calls on arrays of n_rf took 8 us a turn)
+        shifted = False
+        for j in range(rf.n_rf):
+            design = rf.omega_rf_d[j, turn + 1]
+            dphi = rf.dphi_rf[j] + (2.0 * np.pi * rf.harmonic[j, turn + 1]
+                                    * (rf.omega_rf[j, turn + 1] - design) / design)
+            rf.dphi_rf[j] = dphi
+            shifted = shifted or dphi != 0
+        if shifted:
             rf.phi_rf[:, turn + 1] += rf.dphi_rf
             self._sync_phase(turn + 1)
         if not rf.empty:
