@@ -21,6 +21,8 @@ namespace bb {
 
 constexpr int kBatchChunkDefault = 32768;
 constexpr int kBatchMaxThreads = 1024;
+// Launch shapes that the autotuner times again after one turn of each.
+constexpr size_t kBatchFinalists = 8;
 // Largest histogram + table copy per block (four 256-thread blocks per SM
 // stay resident).
 constexpr size_t kBatchTableSmem = 48 * 1024;
@@ -136,11 +138,6 @@ particle_kernel_batch(const BatchArgs a) {
         }
         pa.err = a.err;
         const double cl = a.cut_left[b], iw = a.inv_w[b];
-        // PPT particles per thread and iteration (i + q * blockDim), all
-        // loads issued before any arithmetic (two per thread left ~16 KB of
-        // loads in flight per SM, which capped HBM near 2.4 TB/s).  Whole
-        // warps iterate together, so the aggregated deposit's warp vote
-        // sees every lane.
         // PPT particles per thread and iteration as PPT / 2 pairs of
         // neighbours (one 16-byte dt load, one pair-sized dE load each), all
         // loads issued before any arithmetic (two particles per thread left
@@ -148,7 +145,9 @@ particle_kernel_batch(const BatchArgs a) {
         // Pairs start on an even particle index; an odd first particle and
         // an unpaired last one go through the same arithmetic below.  Whole
         // warps iterate together, so the aggregated deposit's warp vote sees
-        // every lane.
+        // every lane.  FULL: every lane has all its pairs and deposits are
+        // plain, with no test but the bin's (with the F32P64 floors by
+        // addition, 101 -> 91 instructions a particle).
         using E2 = typename Vec2<E>::type;
         constexpr int PP = PPT / 2;
         const int bd = blockDim.x;
@@ -156,9 +155,10 @@ particle_kernel_batch(const BatchArgs a) {
         const int head = (int)(start & 1);
         const long long p0 = (start + head) >> 1;  // first pair
         const int npair = (count - head) >> 1;
-        const double2* dt2 = reinterpret_cast<const double2*>(dt);
-        const E2* dE2 = reinterpret_cast<const E2*>(dE);
-        for (int w = lane_base; w < npair; w += PP * bd) {
+        double2* const dt2 = reinterpret_cast<double2*>(dt) + p0;
+        E2* const dE2 = reinterpret_cast<E2*>(dE) + p0;
+        auto step = [&](int w, auto full) {
+            constexpr bool FULL = decltype(full)::value;
             const int j = w + (threadIdx.x & 31);
             // F32P64: thread 0 prefetches the block's next iteration into L2
             // (C3: 2.059 -> 2.040 ms per turn)
@@ -173,8 +173,8 @@ particle_kernel_batch(const BatchArgs a) {
             bool in[PP];
 #pragma unroll
             for (int q = 0; q < PP; ++q) {
-                in[q] = j + q * bd < npair;
-                const long long g = p0 + (in[q] ? j + q * bd : 0);
+                in[q] = FULL || j + q * bd < npair;
+                const unsigned g = in[q] ? j + q * bd : 0;
                 tq[q] = stream_load(dt2 + g, pol);
                 e[q] = stream_load(dE2 + g, pol);
             }
@@ -186,16 +186,17 @@ particle_kernel_batch(const BatchArgs a) {
 #pragma unroll
                 for (int q = 0; q < PP; ++q) {
                     if (in[q]) {
-                        stream_store(reinterpret_cast<double2*>(dt) + p0 + j + q * bd, tq[q], pol);
-                        stream_store(reinterpret_cast<E2*>(dE) + p0 + j + q * bd, e[q], pol);
+                        const unsigned g = j + q * bd;
+                        stream_store(dt2 + g, tq[q], pol);
+                        stream_store(dE2 + g, e[q], pol);
                     }
                 }
             }
 #pragma unroll
             for (int q = 0; q < PP; ++q) {
-                const int b0 = in[q] ? engine_bin(tq[q].x, cl, iw, S) : -1;
-                const int b1 = in[q] ? engine_bin(tq[q].y, cl, iw, S) : -1;
-                if (a.agg) {
+                const int b0 = in[q] ? engine_bin<PREC == PREC_F32P64>(tq[q].x, cl, iw, S) : -1;
+                const int b1 = in[q] ? engine_bin<PREC == PREC_F32P64>(tq[q].y, cl, iw, S) : -1;
+                if (!FULL && a.agg) {
                     deposit(sh, b0, true, 0xffffffffu);
                     deposit(sh, b1, true, 0xffffffffu);
                 } else {
@@ -203,7 +204,59 @@ particle_kernel_batch(const BatchArgs a) {
                     if (b1 >= 0) atomicAdd(&sh[b1], 1);
                 }
             }
+        };
+        int w = lane_base;
+        const int last = 31 + (PP - 1) * bd;  // a full iteration's last pair from w
+        if constexpr (KICK && PP <= 2) {
+            // Register pipeline: an iteration's loads are issued while the one
+            // before is computed.  With 8 particles a thread the block loads,
+            // then computes (64 registers hold no second set), and on long
+            // runs the chip's power limit, not HBM, sets the rate: 256 beams,
+            // 2.9e8 particles, F32P64, two harmonics: 1410 us a turn with 8
+            // and no pipeline, 1320 with 4 and this one (1470 without it);
+            // 4.9 -> 5.2 TB/s.
+            double2 tn[PP];
+            E2 en[PP];
+            if (!a.agg && w + last < npair) {
+                const int j = w + (threadIdx.x & 31);
+#pragma unroll
+                for (int q = 0; q < PP; ++q) {
+                    tn[q] = stream_load(dt2 + (unsigned)(j + q * bd), pol);
+                    en[q] = stream_load(dE2 + (unsigned)(j + q * bd), pol);
+                }
+                for (; w + last < npair; w += PP * bd) {
+                    const int i = w + (threadIdx.x & 31);
+                    double2 tq[PP];
+                    E2 e[PP];
+#pragma unroll
+                    for (int q = 0; q < PP; ++q) {
+                        tq[q] = tn[q];
+                        e[q] = en[q];
+                    }
+                    if (w + PP * bd + last < npair) {
+#pragma unroll
+                        for (int q = 0; q < PP; ++q) {
+                            tn[q] = stream_load(dt2 + (unsigned)(i + (PP + q) * bd), pol);
+                            en[q] = stream_load(dE2 + (unsigned)(i + (PP + q) * bd), pol);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < PP; ++q) {
+                        track_pair<PREC, SOLVER, LIK, (TSM && LIK) ? TAB_ENTRIES : TAB_GLOBAL,
+                                   true>(tq[q].x, tq[q].y, e[q].x, e[q].y, c, pa, a.order, stab);
+                        stream_store(dt2 + (unsigned)(i + q * bd), tq[q], pol);
+                        stream_store(dE2 + (unsigned)(i + q * bd), e[q], pol);
+                        const int b0 = engine_bin<PREC == PREC_F32P64>(tq[q].x, cl, iw, S);
+                        const int b1 = engine_bin<PREC == PREC_F32P64>(tq[q].y, cl, iw, S);
+                        if (b0 >= 0) atomicAdd(&sh[b0], 1);
+                        if (b1 >= 0) atomicAdd(&sh[b1], 1);
+                    }
+                }
+            }
+        } else if (!a.agg) {
+            for (; w + last < npair; w += PP * bd) step(w, std::true_type{});
         }
+        for (; w < npair; w += PP * bd) step(w, std::false_type{});
         // the odd first particle (thread 0) and the unpaired last one (thread 1)
         if (threadIdx.x < 2 && (threadIdx.x == 0 ? head : (count - head) & 1)) {
             const long long g = threadIdx.x == 0 ? start : start + count - 1;
@@ -215,7 +268,7 @@ particle_kernel_batch(const BatchArgs a) {
                 dt[g] = t0;
                 dE[g] = e0;
             }
-            const int bq = engine_bin(t0, cl, iw, S);
+            const int bq = engine_bin<PREC == PREC_F32P64>(t0, cl, iw, S);
             if (bq >= 0) atomicAdd(&sh[bq], 1);
         }
         __syncthreads();
@@ -777,7 +830,8 @@ int blond_batch_set_shape(blond_batch* q, int threads, int blocks_per_sm,
 }
 
 // Time every launch shape of the particle pass on the bound beams (CUDA
-// events, one warm-up + reps launches each, the coordinates and histograms
+// events; one launch each on large batches, else a warm-up and reps; then
+// twice reps launches of the fastest few; the coordinates and histograms
 // restored afterwards) and keep the fastest.  config receives {threads,
 // blocks_per_sm, particles_per_thread, chunk, aggregate, candidates}.
 int blond_batch_autotune(blond_batch* q, int reps, void* stream, int* config,
@@ -821,26 +875,47 @@ int blond_batch_autotune(blond_batch* q, int reps, void* stream, int* config,
     cudaEventCreate(&b);
     double best = 1e30;
     Cand win = old;
-    for (const Cand& c : cands) {
-        if ((rc = blond_batch_set_shape(q, c.threads, c.bps, c.ppt, c.chunk, c.agg))) break;
-        if ((rc = launch_batch(q, true, s, false))) break;
-        if ((rc = launch_batch(q, true, s))) break;  // warm-up
+    const bool large = n >= (size_t)1 << 23;
+    // `turns` turns of a candidate, in ms per turn
+    auto time_shape = [&](const Cand& c, int turns, double* ms_turn) {
+        int rc = blond_batch_set_shape(q, c.threads, c.bps, c.ppt, c.chunk, c.agg);
+        if (rc == BLOND_OK) rc = launch_batch(q, true, s, false);  // loads the kernel
+        if (rc == BLOND_OK && !large) rc = launch_batch(q, true, s);  // warm-up
         cudaEventRecord(a, s);
-        for (int r = 0; r < reps && rc == BLOND_OK; ++r) rc = launch_batch(q, true, s);
+        for (int r = 0; r < turns && rc == BLOND_OK; ++r) rc = launch_batch(q, true, s);
         cudaEventRecord(b, s);
-        if (rc) break;
+        if (rc) return rc;
         if (cudaEventSynchronize(b) != cudaSuccess) {
             set_error("batch_autotune: a candidate failed");
-            rc = BLOND_ERR_CUDA;
-            break;
+            return (int)BLOND_ERR_CUDA;
         }
         float ms = 0.f;
         cudaEventElapsedTime(&ms, a, b);
-        if (ms / reps < best) {
-            best = ms / reps;
-            win = c;
-        }
+        *ms_turn = ms / turns;
+        return (int)BLOND_OK;
+    };
+    // Every candidate once (one turn of a large batch), then the fastest ones
+    // again, in turn: on large batches the power limit lowers the clocks while
+    // the candidates run, so that times far apart do not compare.
+    std::vector<std::pair<double, int>> order;
+    for (size_t k = 0; k < cands.size() && rc == BLOND_OK; ++k) {
+        double ms = 0.0;
+        rc = time_shape(cands[k], large ? 1 : reps, &ms);
+        if (rc == BLOND_OK) order.push_back({ms, (int)k});
     }
+    std::sort(order.begin(), order.end());
+    if (order.size() > kBatchFinalists) order.resize(kBatchFinalists);
+    std::vector<double> total(order.size(), 0.0);
+    for (int round = 0; round < 2 && rc == BLOND_OK; ++round)
+        for (size_t k = 0; k < order.size() && rc == BLOND_OK; ++k) {
+            double ms = 0.0;
+            rc = time_shape(cands[order[k].second], reps, &ms);
+            total[k] += ms / 2;
+            if (rc == BLOND_OK && round == 1 && total[k] < best) {
+                best = total[k];
+                win = cands[order[k].second];
+            }
+        }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     // restore the state of the run

@@ -219,7 +219,7 @@ __device__ __forceinline__ void rf_sincos(double x, double* sp, double* cp) {
 // (gen_sin_coeffs.py; within 2 float ulps).  No branch.
 __device__ __forceinline__ float rf_sinf(double x) {
     const double shifter = kSin[0];  // 1.5 * 2^52
-    const double ks = __dadd_rn(__dmul_rn(x, kSin[1]), shifter);
+    const double ks = __fma_rn(x, kSin[1], shifter);
     const double k = __dsub_rn(ks, shifter);
     const float r = (float)fma(-k, kSin[13], x);
     const float r2 = r * r;

@@ -247,6 +247,18 @@ __device__ __forceinline__ void rf_sum_pair(const TurnConsts& c, int n_rf, doubl
     }
 }
 
+// floor(y) + 1.5 * 2^52, by one addition that rounds down: for |y| < 2^51 the
+// sum's low word is floor(y), and floor(y) is in [0, 2^32) exactly when its high
+// word is the shifter's own.  NaN, infinities and larger values have other high
+// words.  (A conversion to an integer goes through the quarter-rate conversion
+// unit, 40 % busy in the batched F32P64 pass, and for a bin a NaN test in
+// doubles comes on top.)
+__device__ __forceinline__ double floor_shift(double y) { return __dadd_rd(y, kSin[0]); }
+// floor(y) in [0, n), from floor_shift(y).
+__device__ __forceinline__ bool shifted_below(double ys, int n) {
+    return __double2hiint(ys) == 0x43380000 && (unsigned)__double2loint(ys) < (unsigned)n;
+}
+
 // The interpolation-table entries of two particles: gathered, in range or not,
 // and for F32P64 the offsets from the slice centres.
 template <int PREC>
@@ -259,22 +271,28 @@ struct PairTable {
 template <int PREC, int TAB>
 __device__ __forceinline__ void lookup_pair(double t0, double t1, const ParticleArgs& a,
                                             const void* stab, PairTable<PREC>& p) {
-    // floor(y) in [0, S - 2] exactly when y is in [0, S - 1); the
-    // round-down conversion saturates outside the int range, so one
-    // unsigned compare tests it.  (A NaN y converts to 0 and takes
-    // entry 0; its particle's energy is NaN from the RF kick anyway.)
     const double y0 = (t0 - a.bc0) * a.lik_inv_w;
     const double y1 = (t1 - a.bc0) * a.lik_inv_w;
-    const int r0 = __double2int_rd(y0), r1 = __double2int_rd(y1);
-    p.in0 = (unsigned)r0 < (unsigned)(a.S - 1);
-    p.in1 = (unsigned)r1 < (unsigned)(a.S - 1);
-    const int k0 = p.in0 ? r0 : 0, k1 = p.in1 ? r1 : 0;
-    p.tb0 = table_at<PREC, TAB>(a, stab, k0);
-    p.tb1 = table_at<PREC, TAB>(a, stab, k1);
-    if (PREC == PREC_F32P64) {
+    if constexpr (PREC == PREC_F32P64) {
+        const double m0 = floor_shift(y0), m1 = floor_shift(y1);
+        p.in0 = shifted_below(m0, a.S - 1);
+        p.in1 = shifted_below(m1, a.S - 1);
+        p.tb0 = table_at<PREC, TAB>(a, stab, p.in0 ? __double2loint(m0) : 0);
+        p.tb1 = table_at<PREC, TAB>(a, stab, p.in1 ? __double2loint(m1) : 0);
         // offsets from the slice centre, needed before t changes
-        p.x0f = (float)(t0 - (a.bc0 + (double)k0 * a.bw));
-        p.x1f = (float)(t1 - (a.bc0 + (double)k1 * a.bw));
+        p.x0f = (float)(t0 - (a.bc0 + __dsub_rn(m0, kSin[0]) * a.bw));
+        p.x1f = (float)(t1 - (a.bc0 + __dsub_rn(m1, kSin[0]) * a.bw));
+    } else {
+        // Here the FP64 pipe is the busy one: floor(y) in [0, S - 2] exactly
+        // when y is in [0, S - 1), and the round-down conversion saturates
+        // outside the int range, so one unsigned compare tests it.  (A NaN y
+        // converts to 0 and takes entry 0; its particle's energy is NaN from
+        // the RF kick anyway.)
+        const int r0 = __double2int_rd(y0), r1 = __double2int_rd(y1);
+        p.in0 = (unsigned)r0 < (unsigned)(a.S - 1);
+        p.in1 = (unsigned)r1 < (unsigned)(a.S - 1);
+        p.tb0 = table_at<PREC, TAB>(a, stab, p.in0 ? r0 : 0);
+        p.tb1 = table_at<PREC, TAB>(a, stab, p.in1 ? r1 : 0);
     }
 }
 
@@ -373,11 +391,18 @@ __device__ __forceinline__ void track_pair(double& t0, double& t1,
     track_pair_with<PREC, SOLVER, LIK, RF2>(t0, t1, e0, e1, c, a, order, p);
 }
 
+// The slice of a particle, or -1.  SHIFT: the floor by floor_shift, for passes
+// in which the conversion unit is busier than the FP64 pipe; the same slice.
+template <bool SHIFT = false>
 __device__ __forceinline__ int engine_bin(double t, double cut_left, double inv_w, int S) {
+    const double y = __dmul_rn(__dsub_rn(t, cut_left), inv_w);
+    if constexpr (SHIFT) {
+        const double m = floor_shift(y);
+        return shifted_below(m, S) ? __double2loint(m) : -1;
+    }
     // floor(y) in [0, S) exactly when y is in [0, S); the round-down
     // conversion saturates outside the int range and gives 0 for NaN,
     // which the y == y test excludes
-    const double y = __dmul_rn(__dsub_rn(t, cut_left), inv_w);
     const int k = __double2int_rd(y);
     return ((unsigned)k < (unsigned)S && y == y) ? k : -1;
 }
@@ -633,8 +658,8 @@ particle_kernel(const ParticleArgs a) {
                     stream_store(reinterpret_cast<double2*>(dt) + p, tt, pol);
                     stream_store(reinterpret_cast<E2*>(dE) + p, ee, pol);
                 }
-                b0 = engine_bin(tt.x, a.cut_left, a.inv_w, a.S);
-                b1 = engine_bin(tt.y, a.cut_left, a.inv_w, a.S);
+                b0 = engine_bin<PREC == PREC_F32P64>(tt.x, a.cut_left, a.inv_w, a.S);
+                b1 = engine_bin<PREC == PREC_F32P64>(tt.y, a.cut_left, a.inv_w, a.S);
             }
             if (!a.no_deposit) {
                 deposit(hd, b0, WARP_AGG, 0xffffffffu);
@@ -686,8 +711,8 @@ particle_kernel(const ParticleArgs a) {
                 track_pair<PREC, SOLVER, LIK>(tt.x, tt.y, ee.x, ee.y, c, a, order);
                 stream_store(reinterpret_cast<double2*>(dt) + p, tt, pol);
                 stream_store(reinterpret_cast<E2*>(dE) + p, ee, pol);
-                b0 = engine_bin(tt.x, a.cut_left, a.inv_w, a.S);
-                b1 = engine_bin(tt.y, a.cut_left, a.inv_w, a.S);
+                b0 = engine_bin<PREC == PREC_F32P64>(tt.x, a.cut_left, a.inv_w, a.S);
+                b1 = engine_bin<PREC == PREC_F32P64>(tt.y, a.cut_left, a.inv_w, a.S);
             }
             if (!a.no_deposit) {
                 deposit(hd, b0, WARP_AGG, 0xffffffffu);
@@ -706,7 +731,7 @@ particle_kernel(const ParticleArgs a) {
             dt[a.n - 1] = t;
             dE[a.n - 1] = e;
         }
-        const int b = engine_bin(t, a.cut_left, a.inv_w, a.S);
+        const int b = engine_bin<PREC == PREC_F32P64>(t, a.cut_left, a.inv_w, a.S);
         if (b >= 0 && !a.no_deposit) atomicAdd(&hd[b], 1);
     }
     if (!a.global_hist) cluster_flush(sh, a.hist, a.S);
@@ -762,7 +787,7 @@ particle_kernel_multi(const ParticleArgs a, int first, int n_sub, int deposit_la
     const int64_t npairs = a.n / 2;
     const uint64_t pol = evict_first_policy();
     auto slice = [&](double t) {
-        const int b = engine_bin(t, a.cut_left, a.inv_w, a.S);
+        const int b = engine_bin<PREC == PREC_F32P64>(t, a.cut_left, a.inv_w, a.S);
         if (b >= 0) atomicAdd(&hd[b], 1);
     };
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npairs;
@@ -902,8 +927,8 @@ particle_kernel_stab(const ParticleArgs a) {
                 track_pair<PREC, SOLVER, true, TAB>(tt.x, tt.y, ee.x, ee.y, c, a, order, stab);
                 stream_store(reinterpret_cast<double2*>(dt) + p, tt, pol);
                 stream_store(reinterpret_cast<E2*>(dE) + p, ee, pol);
-                b0 = engine_bin(tt.x, a.cut_left, a.inv_w, S);
-                b1 = engine_bin(tt.y, a.cut_left, a.inv_w, S);
+                b0 = engine_bin<PREC == PREC_F32P64>(tt.x, a.cut_left, a.inv_w, S);
+                b1 = engine_bin<PREC == PREC_F32P64>(tt.y, a.cut_left, a.inv_w, S);
             }
             deposit2(b0, b1, tested);
         };
@@ -949,8 +974,8 @@ particle_kernel_stab(const ParticleArgs a) {
                 track_pair<PREC, SOLVER, true, TAB>(tt.x, tt.y, ee.x, ee.y, c, a, order, stab);
                 stream_store(reinterpret_cast<double2*>(dt) + p, tt, pol);
                 stream_store(reinterpret_cast<E2*>(dE) + p, ee, pol);
-                b0 = engine_bin(tt.x, a.cut_left, a.inv_w, S);
-                b1 = engine_bin(tt.y, a.cut_left, a.inv_w, S);
+                b0 = engine_bin<PREC == PREC_F32P64>(tt.x, a.cut_left, a.inv_w, S);
+                b1 = engine_bin<PREC == PREC_F32P64>(tt.y, a.cut_left, a.inv_w, S);
             }
             deposit2(b0, b1, tested);
             slot = slot + 1 == NST ? 0 : slot + 1;
@@ -968,7 +993,7 @@ particle_kernel_stab(const ParticleArgs a) {
         track_one<PREC, SOLVER, true, true, true, false, TAB>(t, e, c, a, nullptr, order, stab);
         dt[a.n - 1] = t;
         dE[a.n - 1] = e;
-        deposit_packed(sh, half, a.hist, engine_bin(t, a.cut_left, a.inv_w, S));
+        deposit_packed(sh, half, a.hist, engine_bin<PREC == PREC_F32P64>(t, a.cut_left, a.inv_w, S));
     }
     __syncthreads();
     for (int k = threadIdx.x; k < half; k += blockDim.x) {
@@ -1041,8 +1066,8 @@ particle_kernel_pipe(const ParticleArgs a) {
         track_pair_with<PREC, SOLVER, true>(t.x, t.y, e.x, e.y, c, a, a.order, p);
         stream_store(dt + i, t, pol);
         stream_store(dE + i, e, pol);
-        deposit_packed(sh, half, a.hist, engine_bin(t.x, a.cut_left, a.inv_w, S));
-        deposit_packed(sh, half, a.hist, engine_bin(t.y, a.cut_left, a.inv_w, S));
+        deposit_packed(sh, half, a.hist, engine_bin<PREC == PREC_F32P64>(t.x, a.cut_left, a.inv_w, S));
+        deposit_packed(sh, half, a.hist, engine_bin<PREC == PREC_F32P64>(t.y, a.cut_left, a.inv_w, S));
         t = tn;
         e = en;
         tn = t2;
@@ -1058,7 +1083,7 @@ particle_kernel_pipe(const ParticleArgs a) {
         track_one<PREC, SOLVER, true, true, true, false, TAB_GLOBAL>(x, y, c, a, nullptr, a.order);
         *d = x;
         *q = y;
-        deposit_packed(sh, half, a.hist, engine_bin(x, a.cut_left, a.inv_w, S));
+        deposit_packed(sh, half, a.hist, engine_bin<PREC == PREC_F32P64>(x, a.cut_left, a.inv_w, S));
     }
     __syncthreads();
     for (int k = threadIdx.x; k < half; k += blockDim.x) {
@@ -1191,9 +1216,9 @@ particle_kernel_tma(const ParticleArgs a, int* err) {
                 stream_store(reinterpret_cast<E2*>(dE + base) + p, ee, pol);
                 if (!a.no_deposit) {
                     block_deposit<HIST>(sh, half, a.hist,
-                                        engine_bin(tt.x, a.cut_left, a.inv_w, a.S));
+                                        engine_bin<PREC == PREC_F32P64>(tt.x, a.cut_left, a.inv_w, a.S));
                     block_deposit<HIST>(sh, half, a.hist,
-                                        engine_bin(tt.y, a.cut_left, a.inv_w, a.S));
+                                        engine_bin<PREC == PREC_F32P64>(tt.y, a.cut_left, a.inv_w, a.S));
                 }
             }
         }
@@ -1221,7 +1246,7 @@ particle_kernel_tma(const ParticleArgs a, int* err) {
             track_one<PREC, SOLVER, LIK, true, true, false>(t, e, c, a, sh, order);
             dt[i] = t;
             dE[i] = e;
-            const int b = a.no_deposit ? -1 : engine_bin(t, a.cut_left, a.inv_w, a.S);
+            const int b = a.no_deposit ? -1 : engine_bin<PREC == PREC_F32P64>(t, a.cut_left, a.inv_w, a.S);
             if (HIST == HIST_PACKED)
                 deposit_packed(reinterpret_cast<unsigned*>(sh), half, a.hist, b);
             else if (b >= 0)
