@@ -507,6 +507,24 @@ static int launch_particles_range(blond_engine* e, int64_t off, int64_t cnt,
 // accumulator into the float64 profile and zeroes it.
 constexpr int kSmoothThreads = 512;
 
+// The end of a block whose deposits are in `acc`: the last block converts.
+__device__ __forceinline__ void smooth_profile_when_last(unsigned long long* acc,
+                                                         double* profile, int* ticket, int S,
+                                                         int bits) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int k = threadIdx.x; k < S; k += blockDim.x) {
+        const long long v = (long long)atomicExch(&acc[k], 0ull);
+        profile[k] = ldexp((double)v, -bits);
+    }
+    if (threadIdx.x == 0) *ticket = 0;
+}
+
 __global__ void __launch_bounds__(kSmoothThreads)
 smooth_deposit_kernel(const double* __restrict__ dt, int64_t n, double cut_left, double inv_w,
                       double lo, double hi, int S, int bits, int use_smem,
@@ -526,22 +544,11 @@ smooth_deposit_kernel(const double* __restrict__ dt, int64_t n, double cut_left,
         if (k >= 0) atomicAdd(&dst[k], (unsigned long long)llrint(ldexp(w1, bits)));
         if (k2 >= 0) atomicAdd(&dst[k2], (unsigned long long)llrint(ldexp(w2, bits)));
     }
-    __shared__ bool last;
     __syncthreads();
     if (use_smem)
         for (int k = threadIdx.x; k < S; k += blockDim.x)
             if (sacc[k]) atomicAdd(&acc[k], sacc[k]);
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int k = threadIdx.x; k < S; k += blockDim.x) {
-        const long long v = (long long)atomicExch(&acc[k], 0ull);
-        profile[k] = ldexp((double)v, -bits);
-    }
-    if (threadIdx.x == 0) *ticket = 0;
+    smooth_profile_when_last(acc, profile, ticket, S, bits);
 }
 
 static int smooth_bits_for(int64_t n) {
@@ -573,6 +580,164 @@ static int launch_smooth_deposit(blond_engine* e, cudaStream_t s) {
         e->d_profile, e->d_smooth_ticket);
     BB_LAUNCH_CHECK();
     return BLOND_OK;
+}
+
+// The turn's particle pass and its smooth deposit in one launch: the weights
+// are taken from the new dt while it is in registers, so dt is not read a
+// second time and a turn is two launches, chained like the others (programmatic
+// dependent launch).  The sums are smooth_deposit_kernel's, to the bit, but per
+// block in two 32-bit words a slice, the carry passed on by the thread that
+// sees it: a 64-bit shared atomic is a compare-and-swap loop (1e6 particles, 600
+// slices: 10.4 us for the deposit alone, most of it in those loops).  Bound:
+// the pass's FP64 arithmetic on short beams, HBM and the four shared atomics a
+// particle on long ones; each thread loads its next pair before it computes
+// one.  Turns, two kernels -> this one: 1e6 particles, exact drift, 600 slices
+// 23.8 -> 18.9 us; 1e7, 4096 slices 115 -> 76; 1e7 F32P64, 20000 slices 191 -> 99;
+// 2e4 10.1 -> 9.5.
+template <int PREC, int SOLVER, bool LIK>
+__global__ void __launch_bounds__(kEngineThreads, 1)
+particle_kernel_smooth(const ParticleArgs a, double lo, double hi, double scale, int bits,
+                       unsigned long long* __restrict__ acc, double* __restrict__ profile,
+                       int* __restrict__ ticket) {
+    using E = typename Coord<PREC>::E;
+    using E2 = typename Vec2<E>::type;
+    extern __shared__ __align__(16) unsigned ssm[];
+    __shared__ TurnConsts c;
+    pdl_launch_dependents();
+    const int S = a.S;
+    unsigned* const slo = ssm;
+    unsigned* const shi = ssm + S;
+    for (int k = threadIdx.x; k < 2 * S; k += blockDim.x) ssm[k] = 0u;
+    pdl_wait();  // the head's table and turn counter; it has read the profile
+    long long t_idx = a.turn ? (*a.turn - 1) : 0;
+    if (t_idx < 0) t_idx = 0;
+    if (t_idx >= a.n_turns) t_idx = a.n_turns - 1;
+    for (int j = threadIdx.x; j < a.n_rf; j += blockDim.x) {
+        c.V[j] = a.V[t_idx * a.n_rf + j];
+        c.Vf[j] = (float)c.V[j];
+        c.op[j] = make_double2(a.om[t_idx * a.n_rf + j], a.ph[t_idx * a.n_rf + j]);
+    }
+    if (threadIdx.x == 0) {
+        c.acc = a.interp ? 0.0 : a.acc[t_idx];
+        c.d = a.drift[t_idx + 1];
+    }
+    __syncthreads();
+    auto add = [&](int k, double w) {
+        if (k < 0) return;
+        const long long v = __double2ll_rn(w * scale);
+        const unsigned low = (unsigned)v;
+        unsigned high = (unsigned)((unsigned long long)v >> 32);
+        const unsigned old = atomicAdd(&slo[k], low);
+        if (old + low < old) ++high;
+        if (high) atomicAdd(&shi[k], high);
+    };
+    auto slice = [&](double t) {
+        int k, k2;
+        double w1 = 0.0, w2 = 0.0;
+        smooth_weights<double>(t, a.cut_left, a.inv_w, lo, hi, S, k, k2, w1, w2);
+        add(k, w1);
+        add(k2, w2);
+    };
+    double2* const dt = reinterpret_cast<double2*>(a.dt);
+    E2* const dE = reinterpret_cast<E2*>(a.dE);
+    const int64_t npairs = a.n / 2;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const uint64_t pol = evict_first_policy();
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double2 tn;
+    E2 en;
+    if (i < npairs) {
+        tn = stream_load(dt + i, pol);
+        en = stream_load(dE + i, pol);
+    }
+    for (; i < npairs; i += stride) {
+        double2 t = tn;
+        E2 e = en;
+        if (i + stride < npairs) {
+            tn = stream_load(dt + i + stride, pol);
+            en = stream_load(dE + i + stride, pol);
+        }
+        track_pair<PREC, SOLVER, LIK>(t.x, t.y, e.x, e.y, c, a, a.order);
+        stream_store(dt + i, t, pol);
+        stream_store(dE + i, e, pol);
+        slice(t.x);
+        slice(t.y);
+    }
+    // odd tail particle
+    if ((a.n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        double* const d = reinterpret_cast<double*>(a.dt) + a.n - 1;
+        E* const q = reinterpret_cast<E*>(a.dE) + a.n - 1;
+        double x = *d;
+        E y = *q;
+        track_one<PREC, SOLVER, LIK, true, true, false>(x, y, c, a, nullptr, a.order);
+        *d = x;
+        *q = y;
+        slice(x);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < S; k += blockDim.x) {
+        const unsigned long long v = ((unsigned long long)shi[k] << 32) + slo[k];
+        if (v) atomicAdd(&acc[k], v);
+    }
+    smooth_profile_when_last(acc, profile, ticket, S, bits);
+}
+
+// Dynamic shared memory of the pass with its own smooth deposit, or -1 when the
+// two words a slice do not fit (about 28000 slices) or the options name a pass
+// that launch_particles refuses: the particle pass and smooth_deposit_kernel
+// then follow each other.
+static int smooth_pass_smem(const blond_engine* e) {
+    if (!e->smooth || e->variant == 2 || e->variant == 3) return -1;
+    if (e->ring && (e->precision == BLOND_PREC_F64 ? plain_ring_smem<PREC_F64>(e, e->ring)
+                                                   : plain_ring_smem<PREC_F32P64>(e, e->ring)) < 0)
+        return -1;
+    const size_t bytes = 8 * (size_t)e->S;
+    const size_t limit = (size_t)device_info().max_smem_optin - sizeof(TurnConsts) - 1024;
+    return bytes <= limit ? (int)bytes : -1;
+}
+
+template <int PREC, int SOLVER>
+static int launch_smooth_pass_k(blond_engine* e, cudaStream_t s, bool launch) {
+    const bool lik = e->has_fft || e->has_ind || e->interp;
+    auto k = lik ? particle_kernel_smooth<PREC, SOLVER, true>
+                 : particle_kernel_smooth<PREC, SOLVER, false>;
+    const int rc = allow_smem_once(k);
+    if (rc) return rc;
+    if (!launch) return BLOND_OK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(particle_grid(e->n / 2 + 1, kEngineThreads, 1), 1, 1);
+    cfg.blockDim = dim3(kEngineThreads, 1, 1);
+    cfg.dynamicSmemBytes = smooth_pass_smem(e);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = e->pdl ? 1 : 0;
+    const double w = (e->cut_right - e->cut_left) / e->S;
+    BB_CUDA(cudaLaunchKernelEx(&cfg, k, particle_args(e), e->cut_left + w * 0.5,
+                               e->cut_right - w * 0.5, std::ldexp(1.0, e->smooth_bits),
+                               e->smooth_bits, reinterpret_cast<unsigned long long*>(e->d_acc64),
+                               e->d_profile, e->d_smooth_ticket));
+    BB_LAUNCH_CHECK();
+    return BLOND_OK;
+}
+
+template <int PREC>
+static int launch_smooth_pass_p(blond_engine* e, cudaStream_t s, bool launch) {
+    switch (e->solver) {
+        case 0: return launch_smooth_pass_k<PREC, 0>(e, s, launch);
+        case 1: return launch_smooth_pass_k<PREC, 1>(e, s, launch);
+        default: return launch_smooth_pass_k<PREC, 2>(e, s, launch);
+    }
+}
+
+static int launch_smooth_pass(blond_engine* e, cudaStream_t s, bool launch = true) {
+    switch (e->precision) {
+        case BLOND_PREC_F64: return launch_smooth_pass_p<PREC_F64>(e, s, launch);
+        case BLOND_PREC_F32P64: return launch_smooth_pass_p<PREC_F32P64>(e, s, launch);
+        default: return launch_smooth_pass_p<PREC_Q32P64>(e, s, launch);
+    }
 }
 
 static int launch_profile(blond_engine* e, bool clear, cudaStream_t s) {
@@ -790,6 +955,7 @@ static int launch_spectral_head(blond_engine* e, cudaStream_t s, bool loop) {
 static int launch_turn(blond_engine* e, cudaStream_t s) {
     int rc = launch_head(e, s);
     if (rc) return rc;
+    if (smooth_pass_smem(e) >= 0) return launch_smooth_pass(e, s);
     if ((rc = launch_particles(e, true, s))) return rc;
     return e->smooth ? launch_smooth_deposit(e, s) : BLOND_OK;
 }
@@ -1304,6 +1470,7 @@ namespace bb {
 static int time_graph_turns(blond_engine* e, cudaStream_t s, int turns, int reps, double* ms) {
     int rc;
     if ((rc = launch_particles(e, true, s, false))) return rc;
+    if (smooth_pass_smem(e) >= 0 && (rc = launch_smooth_pass(e, s, false))) return rc;
     if (e->has_fft && (rc = prepare_spectral())) return rc;
     cudaGraph_t g = nullptr;
     BB_CUDA(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -1609,6 +1776,7 @@ static int ensure_graph(blond_engine* e, cudaStream_t s) {
     int rc;
     // kernel attributes are set here, never inside the capture
     if ((rc = launch_particles(e, true, s, false))) return rc;
+    if (smooth_pass_smem(e) >= 0 && (rc = launch_smooth_pass(e, s, false))) return rc;
     if (e->has_fft && (rc = prepare_spectral())) return rc;
     if (e->graph) cudaGraphExecDestroy(e->graph);
     e->graph = nullptr;
