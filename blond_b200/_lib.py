@@ -63,6 +63,8 @@ _EXTRA = {
     "blond_irfft_f64": [c_ptr, c_i64, c_ptr, c_i64, c_ptr],
     "blond_induced_voltage_f64": [c_ptr, c_int, c_ptr, c_i64, c_dbl, c_ptr,
                                   c_i64, c_ptr],
+    "blond_induced_voltage_f32": [c_ptr, c_int, c_ptr, c_i64, c_dbl, c_ptr,
+                                  c_i64, c_ptr],
     "blond_engine_create": [ct.POINTER(c_ptr), c_int, c_int, c_int, c_int],
     "blond_engine_destroy": [c_ptr],
     "blond_engine_set_rf": [c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_dbl],

@@ -224,19 +224,27 @@ def rfftfreq(n, d=1.0):
     return np.fft.rfftfreq(int(n), d)
 
 
-def induced_voltage_1turn(profile, total_impedance, n_fft, scale, n_out):
+def induced_voltage_1turn(profile, total_impedance, n_fft, scale, n_out,
+                          dtype=torch.float64):
     """-scale * irfft(total_impedance * rfft(profile, n_fft))[:n_out]
-    (impedance.py:475-489) in one launch; float64 tensor of n_out values."""
-    p = as_device(profile, torch.float64)
+    (impedance.py:475-489) in one launch; tensor of n_out values, computed in
+    float64 and rounded to dtype.  float32 objects (profile and dtype) are
+    converted by the transform's own loads and stores: two conversion launches
+    of 3 us fewer, and their host time."""
+    if dtype == torch.float32 and isinstance(profile, torch.Tensor) and \
+            profile.dtype == torch.float32:
+        p, name = as_device(profile, torch.float32), "blond_induced_voltage_f32"
+    else:
+        p, name = as_device(profile, torch.float64), "blond_induced_voltage_f64"
     Z = total_impedance if isinstance(total_impedance, torch.Tensor) else \
         torch.as_tensor(np.asarray(total_impedance, np.complex128),
                         device=p.device)
     if Z.dtype != torch.complex128 or not Z.is_contiguous():
         Z = Z.to(torch.complex128).contiguous()
-    out = torch.empty(int(n_out), dtype=torch.float64, device=p.device)
-    _lib.call("blond_induced_voltage_f64", _ptr(p), p.numel(), _ptr(Z),
+    out = torch.empty(int(n_out), dtype=p.dtype, device=p.device)
+    _lib.call(name, _ptr(p), p.numel(), _ptr(Z),
               int(n_fft), float(scale), _ptr(out), int(n_out), _stream())
-    return out
+    return out if out.dtype == dtype else out.to(dtype)
 
 
 # ------------------------------------------------------------ beam phase

@@ -183,6 +183,9 @@ head_fft_kernel(const SpecParams P) {
                 if (P.in_i32) {
                     if (i < nlim) x[u].x = (double)__ldcg(P.in_i32 + i);
                     if (i + 1 < nlim) x[u].y = (double)__ldcg(P.in_i32 + i + 1);
+                } else if (P.in_f32) {
+                    if (i < nlim) x[u].x = (double)__ldcg(P.in_f32 + i);
+                    if (i + 1 < nlim) x[u].y = (double)__ldcg(P.in_f32 + i + 1);
                 } else {
                     if (i < nlim) x[u].x = __ldcg(P.in_f64 + i);
                     if (i + 1 < nlim) x[u].y = __ldcg(P.in_f64 + i + 1);
@@ -322,8 +325,13 @@ head_fft_kernel(const SpecParams P) {
             const int m1 = lane + 32 * q;
             const int64_t n = 2 * (int64_t)(c * Bc + b + M2 * m1);
             const double2 o = make_double2(value(n, v[q].x), value(n + 1, v[q].y));
-            if (n < P.n_out) P.out[n] = o.x;
-            if (n + 1 < P.n_out) P.out[n + 1] = o.y;
+            if (P.out_f32) {
+                if (n < P.n_out) P.out_f32[n] = (float)o.x;
+                if (n + 1 < P.n_out) P.out_f32[n + 1] = (float)o.y;
+            } else {
+                if (n < P.n_out) P.out[n] = o.x;
+                if (n + 1 < P.n_out) P.out[n + 1] = o.y;
+            }
             if (P.table) {
                 vloc[b * M1 + m1] = o;
                 // the value after the last of the column before: to its CTA

@@ -294,6 +294,30 @@ static int set_direct_attrs() {
     return BLOND_OK;
 }
 
+// P holds the real input and output of either type.
+static int induced_voltage(SpecParams& P, const void* profile, int n_slices,
+                           const double* impedance, int64_t n_fft, double scale, const void* v_out,
+                           int64_t n_out, void* stream) {
+    BB_CHECK_ARG(n_slices >= 1 && n_fft >= 1 && n_out >= 0,
+                 "induced_voltage: bad length");
+    BB_CHECK_ARG(profile && impedance && (n_out == 0 || v_out),
+                 "induced_voltage: null pointer");
+    cudaStream_t s = as_stream(stream);
+    if (make_spec_plan(n_fft, P.p)) {
+        P.mode = SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE;
+        P.n_in = n_slices;
+        P.H = reinterpret_cast<const double2*>(impedance);
+        P.n_out = n_out < n_fft ? n_out : n_fft;
+        P.out_scale = -scale / (double)P.p.M;
+        P.twg = shared_twiddles(P.p, s);
+        return launch_spectral(P, s);
+    }
+    set_error("induced_voltage: n_fft=%lld is not an even 5-smooth length <= %lld; "
+              "use blond_rfft_f64/blond_irfft_f64", (long long)n_fft,
+              (long long)kMaxClusterFFT);
+    return BLOND_ERR_UNSUPPORTED;
+}
+
 }  // namespace bb
 
 using namespace bb;
@@ -363,27 +387,20 @@ int blond_induced_voltage_f64(const double* profile, int n_slices,
                               const double* impedance, int64_t n_fft,
                               double scale, double* v_out, int64_t n_out,
                               void* stream) {
-    BB_CHECK_ARG(n_slices >= 1 && n_fft >= 1 && n_out >= 0,
-                 "induced_voltage: bad length");
-    BB_CHECK_ARG(profile && impedance && (n_out == 0 || v_out),
-                 "induced_voltage: null pointer");
-    cudaStream_t s = as_stream(stream);
     SpecParams P = {};
-    if (make_spec_plan(n_fft, P.p)) {
-        P.mode = SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE;
-        P.in_f64 = profile;
-        P.n_in = n_slices;
-        P.H = reinterpret_cast<const double2*>(impedance);
-        P.out = v_out;
-        P.n_out = n_out < n_fft ? n_out : n_fft;
-        P.out_scale = -scale / (double)P.p.M;
-        P.twg = shared_twiddles(P.p, s);
-        return launch_spectral(P, s);
-    }
-    set_error("induced_voltage: n_fft=%lld is not an even 5-smooth length <= %lld; "
-              "use blond_rfft_f64/blond_irfft_f64", (long long)n_fft,
-              (long long)kMaxClusterFFT);
-    return BLOND_ERR_UNSUPPORTED;
+    P.in_f64 = profile;
+    P.out = v_out;
+    return induced_voltage(P, profile, n_slices, impedance, n_fft, scale, v_out, n_out, stream);
+}
+
+int blond_induced_voltage_f32(const float* profile, int n_slices,
+                              const double* impedance, int64_t n_fft,
+                              double scale, float* v_out, int64_t n_out,
+                              void* stream) {
+    SpecParams P = {};
+    P.in_f32 = profile;
+    P.out_f32 = v_out;
+    return induced_voltage(P, profile, n_slices, impedance, n_fft, scale, v_out, n_out, stream);
 }
 
 }  // extern "C"

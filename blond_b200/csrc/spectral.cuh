@@ -75,8 +75,10 @@ enum : int {
 struct SpecParams {
     SpecPlan p;
     int mode;
-    // real input (profile): exactly one of in_f64 / in_i32 is set
+    // real input (profile): exactly one of in_f64 / in_i32 / in_f32 is set
     const double* in_f64;
+    const float* in_f32;  // float32 objects' profile and voltage (out_f32):
+    float* out_f32;       // converted here, the transform itself in float64
     int* in_i32;          // engine histogram; zeroed after it is read
     int64_t n_in;
     double* profile_out;  // engine: converted profile (n_in doubles)
@@ -620,6 +622,9 @@ spectral_kernel(const SpecParams P, const typename SpecLoopArg<FB>::type LP) {
                     if (i0 < nlim) fb_add(fbb, (int)i0, x0, fb_s, fb_c);
                     if (i1 < nlim) fb_add(fbb, (int)i1, x1, fb_s, fb_c);
                 }
+            } else if (P.in_f32) {
+                if (i0 < nlim) x0 = (double)P.in_f32[boff + i0];
+                if (i1 < nlim) x1 = (double)P.in_f32[boff + i1];
             } else {
                 if (i0 < nlim) x0 = g_in_f64[i0];
                 if (i1 < nlim) x1 = g_in_f64[i1];
@@ -817,8 +822,13 @@ spectral_kernel(const SpecParams P, const typename SpecLoopArg<FB>::type LP) {
         const int64_t m = (int64_t)c * Bc + b + (int64_t)M2 * m1;
         const double2 u = cres[m1 * Bc + b];
         const double v0 = value(2 * m, u.x), v1 = value(2 * m + 1, u.y);
-        if (2 * m < P.n_out) g_out[2 * m] = v0;
-        if (2 * m + 1 < P.n_out) g_out[2 * m + 1] = v1;
+        if (P.out_f32) {
+            if (2 * m < P.n_out) P.out_f32[boff + 2 * m] = (float)v0;
+            if (2 * m + 1 < P.n_out) P.out_f32[boff + 2 * m + 1] = (float)v1;
+        } else {
+            if (2 * m < P.n_out) g_out[2 * m] = v0;
+            if (2 * m + 1 < P.n_out) g_out[2 * m + 1] = v1;
+        }
         if (g_table) {
             vloc[e] = v0;
             // v0 is V[2(m-1)+2] for the element before m: hand it to the

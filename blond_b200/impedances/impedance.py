@@ -163,7 +163,7 @@ class _InducedVoltage:
         if _smooth_even(self.n_fft):
             v = bm.induced_voltage_1turn(self.profile.n_macroparticles,
                                          self.total_impedance, self.n_fft,
-                                         self._scale(), self.n_induced_voltage)
+                                         self._scale(), self.n_induced_voltage, dtype)
         else:
             if beam_spectrum_dict is None:
                 beam_spectrum_dict = {}

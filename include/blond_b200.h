@@ -206,6 +206,12 @@ int blond_induced_voltage_f64(const double* profile, int n_slices,
                               const double* impedance, int64_t n_fft,
                               double scale, double* v_out, int64_t n_out,
                               void* stream);
+/* The same of a float32 profile, the voltage rounded to float32: float64 inside,
+ * without conversion passes around it. */
+int blond_induced_voltage_f32(const float* profile, int n_slices,
+                              const double* impedance, int64_t n_fft,
+                              double scale, float* v_out, int64_t n_out,
+                              void* stream);
 
 /* ------------------------------------------------------------ time-domain wakes
  * Analytic resonator convolution of InducedVoltageResonator: replaces
