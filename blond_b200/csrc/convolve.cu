@@ -30,6 +30,10 @@ __device__ __forceinline__ void fill_shared(double* dst, int n, int tid, int nth
 // profile, the beam-phase sums, the ticket that tells when every block has
 // read the histogram, then (last block) the clearing and the loop's turn.  On
 // a computing warp the ticket's round trip alone took 0.7 us of a 4 us launch.
+// The loop is one chain of memory round trips, the longest of the launch: its
+// sums are taken from the histogram itself while the other warps load, and the
+// blocks' sums are fetched while the histogram is cleared (turns of 2e4
+// particles, 2000 slices 13.0 -> 11.8 us; 10.9 without the loop).
 template <bool FB>
 __global__ void __launch_bounds__(kConvThreads + 32)
 conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
@@ -57,29 +61,16 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
     });
     pdl_wait();  // the particle pass: histogram, turn counter, RF programme
     const long long turn = P.turn ? *P.turn : 0;
-    if (P.in_i32) {
-        const int* const in = P.in_i32 + boff;
-        fill_shared(prof, T, tid, nth + 32, [&](int j) { return j < S ? __ldcg(in + j) : 0; });
-    } else if (P.in_fix) {
-        const unsigned long long* const in = P.in_fix + boff;
-        fill_shared(prof, T, tid, nth + 32, [&](int j) {
-            return j < S ? (double)__ldcg(in + j) * P.fix_unit : 0.0;
-        });
-    } else {
-        const double* const in = P.in_f64 + boff;
-        fill_shared(prof, T, tid, nth + 32, [&](int j) { return j < S ? __ldcg(in + j) : 0.0; });
-    }
-    __syncthreads();
-    if (tid >= nth) {
-        if (P.profile_out)
-            for (int o = lane; o < n_own; o += 32) P.profile_out[boff + i0 + o] = prof[i0 + o];
-        if (!P.ticket) return;
-        if constexpr (FB) {
-            // this block's bins of the beam-phase sums
+    if constexpr (FB) {
+        // this block's bins of the beam-phase sums, while the others load
+        if (tid >= nth) {
             double s = 0.0, c = 0.0;
             if (turn >= fb.delay) {
                 const FbBins b = fb_bins(fb, turn);
-                for (int o = lane; o < n_own; o += 32) fb_add(b, i0 + o, prof[i0 + o], s, c);
+                for (int o = lane; o < n_own; o += 32)
+                    fb_add(b, i0 + o,
+                           P.in_i32 ? (double)__ldcg(P.in_i32 + i0 + o) : __ldcg(P.in_f64 + i0 + o),
+                           s, c);
             }
             for (int d = 16; d > 0; d >>= 1) {
                 s += __shfl_down_sync(0xffffffffu, s, d);
@@ -90,6 +81,25 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
                 fb.phase_partials[2 * cta + 1] = c;
             }
         }
+    }
+    const int nfill = FB ? nth : nth + 32;
+    if (P.in_i32) {
+        const int* const in = P.in_i32 + boff;
+        fill_shared(prof, T, tid, nfill, [&](int j) { return j < S ? __ldcg(in + j) : 0; });
+    } else if (P.in_fix) {
+        const unsigned long long* const in = P.in_fix + boff;
+        fill_shared(prof, T, tid, nfill, [&](int j) {
+            return j < S ? (double)__ldcg(in + j) * P.fix_unit : 0.0;
+        });
+    } else {
+        const double* const in = P.in_f64 + boff;
+        fill_shared(prof, T, tid, nfill, [&](int j) { return j < S ? __ldcg(in + j) : 0.0; });
+    }
+    __syncthreads();
+    if (tid >= nth) {
+        if (P.profile_out)
+            for (int o = lane; o < n_own; o += 32) P.profile_out[boff + i0 + o] = prof[i0 + o];
+        if (!P.ticket) return;
         int last = 0;
         if (lane == 0) {
             __threadfence();
@@ -97,6 +107,17 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
         }
         if (!__shfl_sync(0xffffffffu, last, 0)) return;
         __threadfence();
+        // the blocks' sums, on their way while the histogram is cleared
+        constexpr int kSums = 5;  // at most 148 blocks
+        double ps[kSums], pc[kSums];
+        if constexpr (FB) {
+#pragma unroll
+            for (int k = 0; k < kSums; ++k) {
+                const int q = lane + 32 * k;
+                ps[k] = q < P.p.ctas ? __ldcg(fb.phase_partials + 2 * q) : 0.0;
+                pc[k] = q < P.p.ctas ? __ldcg(fb.phase_partials + 2 * q + 1) : 0.0;
+            }
+        }
         // every block has read the histogram and the counter
         if (P.in_i32)
             for (int j = lane; j < S; j += 32) P.in_i32[boff + j] = 0;
@@ -108,7 +129,12 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
         }
         if constexpr (FB) {
             double s = 0.0, c = 0.0;
-            for (int q = lane; q < P.p.ctas; q += 32) {
+#pragma unroll
+            for (int k = 0; k < kSums; ++k) {
+                s += ps[k];
+                c += pc[k];
+            }
+            for (int q = lane + 32 * kSums; q < P.p.ctas; q += 32) {
                 s += __ldcg(fb.phase_partials + 2 * q);
                 c += __ldcg(fb.phase_partials + 2 * q + 1);
             }
