@@ -730,11 +730,12 @@ int blond_batch_set_impedance(blond_batch* q, int64_t n_fft, const double* Z,
     if ((rc = make_spec_twiddles(plan, &q->d_tw))) return rc;
     q->plan = plan;
     q->has_fft = true;
-    // short profiles: the direct convolution's impulse responses
+    // short profiles: the direct convolution's impulse responses (not in
+    // Q32P64, as in blond_engine_set_impedance)
     q->conv = false;
     free_ptr(q->d_hx);
     q->d_hx = nullptr;
-    if (make_conv_plan(q->S, n_fft, q->B, q->cplan)) {
+    if (q->precision != BLOND_PREC_Q32P64 && make_conv_plan(q->S, n_fft, q->B, q->cplan)) {
         for (int b = 0; b < q->B; ++b) sc[b] = -scale[b];
         if ((rc = upload((void**)&q->d_cscale, sc.data(), sizeof(double) * q->B))) return rc;
         if (!q->d_cticket) {

@@ -68,9 +68,10 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
             if (turn >= fb.delay) {
                 const FbBins b = fb_bins(fb, turn);
                 for (int o = lane; o < n_own; o += 32)
-                    fb_add(b, i0 + o,
-                           P.in_i32 ? (double)__ldcg(P.in_i32 + i0 + o) : __ldcg(P.in_f64 + i0 + o),
-                           s, c);
+                    fb_add<true>(b, i0 + o,
+                                 P.in_i32 ? (double)__ldcg(P.in_i32 + i0 + o)
+                                          : __ldcg(P.in_f64 + i0 + o),
+                                 s, c);
             }
             for (int d = 16; d > 0; d >>= 1) {
                 s += __shfl_down_sync(0xffffffffu, s, d);
@@ -252,8 +253,8 @@ bool make_conv_plan(int S, int64_t N, int B, ConvPlan& plan) {
     const bool pow2 = (N & (N - 1)) == 0;
     // one profile: S^2 multiply-adds over all SMs against the FFT's chain of
     // phases (turns of 2e4 particles, FFT -> convolution: 201 slices 16.9 ->
-    // 6.7 us, 1024 12.0 -> 8.0, 2000 24.1 -> 9.6, 4096 13.2 -> 10.8, 8192
-    // 12.8 -> 14.2, 9000 61.6 -> 16.7)
+    // 7.2 us, 1000 19.8 -> 7.8, 2000 24.1 -> 8.6, 4096 13.2 -> 9.9, 8192
+    // 12.8 -> 14.2, 9000 61.6 -> 16.2)
     if (B == 1 && pow2 && S > 4600) return false;
     // a batch: the profiles' multiply-adds share the SMs (37 beams of 400
     // slices 21.2 -> 14.5 us a turn, but 64 of 512 would be 16 -> 23 and 256 of

@@ -913,6 +913,7 @@ static int launch_spectral_head(blond_engine* e, cudaStream_t s, bool loop) {
     P.p = e->plan;
     P.mode = SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE;
     P.pdl = e->pdl ? 1 : 0;
+    P.general = e->precision == BLOND_PREC_Q32P64;
     P.n_in = e->S;
     P.profile_out = e->d_profile;
     if (e->smooth)
@@ -1217,11 +1218,16 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
                   "profile (%d slices)", (long long)n_fft, e->S);
     int rc = upload((void**)&e->d_H, Z, sizeof(double2) * (size_t)(n_fft / 2 + 1));
     if (rc) return rc;
-    // short profiles: the direct convolution's impulse response
+    // Short profiles: the direct convolution's impulse response.  Not in
+    // Q32P64: where its voltages round otherwise in the last bit, a few
+    // energies a million move by a whole count, and a run would no longer
+    // repeat one of an earlier build.  Its head stays the cluster FFT with
+    // that kernel's roundings (2e4 particles, 2000 slices 24 us a turn, 9 with
+    // the convolution; 1e8 particles, 2^16 slices: 1 % of the turn).
     e->conv = false;
     free_ptr(e->d_hx);
     e->d_hx = nullptr;
-    if (make_conv_plan(e->S, n_fft, 1, e->cplan)) {
+    if (e->precision != BLOND_PREC_Q32P64 && make_conv_plan(e->S, n_fft, 1, e->cplan)) {
         if (!e->d_cticket) {
             BB_CUDA(cudaMalloc((void**)&e->d_cticket, sizeof(int)));
             BB_CUDA(cudaMemset(e->d_cticket, 0, sizeof(int)));
@@ -1229,7 +1235,8 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
         if ((rc = make_conv_response(e->d_H, n_fft, e->S, 1, &e->d_hx))) return rc;
         if ((rc = prepare_conv())) return rc;
         e->conv = true;
-    } else if (const int64_t P = head_fft_length(n_fft, e->S)) {
+    } else if (const int64_t P =
+                   e->precision != BLOND_PREC_Q32P64 ? head_fft_length(n_fft, e->S) : 0) {
         // long profiles at other lengths: the same voltages by the
         // power-of-two transform
         double2* H = nullptr;

@@ -108,6 +108,10 @@ __device__ __forceinline__ FbBins fb_bins(const FeedbackArgs& a, long long t) {
 // trapezoid weight within the window (trapz_const_delta,
 // blondmath.cpp:496-512): 1 inside, 1/2 at either end, 1 for a window of
 // one bin, 0 outside.
+// OWN: with rf_sincos, on the short chain of the convolution head; elsewhere
+// CUDA's sincos, whose last bit Q32P64 runs keep (see
+// blond_engine_set_impedance).
+template <bool OWN = false>
 __device__ __forceinline__ void fb_add(const FbBins& b, int i, double x, double& s_sum,
                                        double& c_sum) {
     const double bci = b.bc[i];
@@ -119,7 +123,8 @@ __device__ __forceinline__ void fb_add(const FbBins& b, int i, double x, double&
     const double base =
         b.machine != BLOND_FB_SPS_F && b.alpha != 0.0 ? exp(b.alpha * bci) * x : x;
     double sn, cs;
-    rf_sincos(b.omega * bci + b.phi, &sn, &cs);
+    if constexpr (OWN) rf_sincos(b.omega * bci + b.phi, &sn, &cs);
+    else sincos(b.omega * bci + b.phi, &sn, &cs);
     s_sum += w * (base * sn);
     c_sum += w * (base * cs);
 }

@@ -380,7 +380,7 @@ bool for_shape(int M1, int M2, F f) {
 }  // namespace
 
 bool head_fft_takes(const SpecParams& P) {
-    if (P.mode != (SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE) || P.batch ||
+    if (P.mode != (SPEC_FORWARD | SPEC_MULTIPLY | SPEC_INVERSE) || P.batch || P.general ||
         P.p.C != kHeadCtas || P.n_in > P.p.N || P.n_out > P.p.N)
         return false;
     bool fits = false;

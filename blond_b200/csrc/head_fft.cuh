@@ -15,7 +15,7 @@ int prepare_head_fft();
 // impulse response at lags |d| < S only, which a circular convolution of
 // length P >= 2 S - 1 gives as well.  P when this kernel takes it, else 0
 // (turns of 1e7 FP64 particles, 20000 slices: 116 us with the mixed-radix
-// transform of 20000 points, 91 with this one of 65536).
+// transform of 20000 points, 86 with this one of 65536).
 int64_t head_fft_length(int64_t N, int S);
 // The spectrum (cudaMalloc'd, P / 2 + 1 values) of that response from the
 // impedance H, N / 2 + 1 values on the device.  Synchronous.

@@ -121,6 +121,9 @@ struct SpecParams {
     // the kernel triggers its dependents at entry and waits for the grid
     // before it before reading the histogram or the turn counter
     int pdl;
+    // take spectral_kernel also where the long-profile kernel (head_fft.cu)
+    // applies: Q32P64 engines, which keep this kernel's roundings
+    int general;
 };
 
 // The engine's beam-phase loop run inside the head (single profile only):

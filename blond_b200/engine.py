@@ -168,7 +168,7 @@ class FusedTracker:
             # RF + induced voltage interpolated from one table, no RF kick
             self.eng.call("set_interpolation", 1)
         if getattr(profile, "smooth", False):
-            # slice_smooth weights, deposited after each particle pass
+            # slice_smooth weights, deposited by the particle pass
             self.eng.call("set_smooth", 1)
         self.loop = getattr(tracker, "beamFB", None)
         # coordinates
@@ -350,9 +350,10 @@ class FusedTracker:
     def autotune(self, reps: int = 3) -> dict:
         """Run the engine's autotuner now (blond_engine_autotune): times
         every feasible particle-pass configuration on this beam, keeps the
-        fastest, then whole turns with and without the early launch of each
-        turn's next kernel ('overlap'), and leaves the beam and the turn
-        state untouched.  Returns the choice."""
+        fastest, then whole turns of the nearest kinds of pass with and
+        without the early launch of each turn's next kernel ('overlap'), and
+        leaves the beam and the turn state untouched.  'prefetch_stages' 1 of
+        the packed pass is its register pipeline.  Returns the choice."""
         cfg = (ct.c_int * 9)()
         ms = ct.c_double()
         self.eng.call("autotune", int(reps), _stream(), cfg, ct.byref(ms))

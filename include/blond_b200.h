@@ -336,10 +336,11 @@ int blond_engine_set_energy_unit(blond_engine* engine, double lsb);
  * is an FFT impedance. */
 int blond_engine_set_interpolation(blond_engine* engine, int on);
 /* Profile with OtherSlicesOptions(smooth=True) (beam/profile.py:764-773):
- * each turn ends with a deposit pass of the reference's slice_smooth
- * weights (histogram.cpp:75-132) accumulated in 64-bit fixed point (2^-b
- * per unit weight, b = min(52, 62 - ceil(log2(1.5 n + 2))); the same bits
- * every run), which is the profile the next turn's induced voltage uses.
+ * the particle pass (above about 28000 slices a deposit pass after it)
+ * deposits the reference's slice_smooth weights (histogram.cpp:75-132) in
+ * 64-bit fixed point (2^-b per unit weight, b = min(52, 62 -
+ * ceil(log2(1.5 n + 2))); the same bits every run), which is the profile
+ * the next turn's induced voltage uses.
  * on = 0/1.  Not with a beam-phase loop or a bound (sharded) histogram. */
 int blond_engine_set_smooth(blond_engine* engine, int on);
 int blond_engine_set_turn(blond_engine* engine, int64_t turn, void* stream);
@@ -471,11 +472,13 @@ int blond_engine_set_cluster(blond_engine* engine, int blocks);
 /* Autotuner: times every feasible particle-pass configuration (plain pass:
  * 256/512/1024 threads x 1/2/4 blocks per SM x histogram layouts x prefetch
  * ring 0/2/4 x clusters of 1/2; staged pass: histogram layouts; shared-table
- * pass: ring 0/2; packed-histogram pass: ring 0/2/4) on the bound beam,
- * `reps` (1..10) launches each after one warm-up, and keeps the fastest;
- * then replays a few whole turns with and without programmatic dependent
- * launch (blond_engine_set_overlap) and keeps the faster (not with a
- * beam-phase loop or smooth slicing).  Restores the coordinates, the
+ * pass: ring 0/2; packed-histogram pass: ring 0/2/4, or 1 for loads one
+ * iteration ahead in registers) on the bound beam, `reps` (1..10) launches
+ * each after one warm-up; then replays a few whole turns with the fastest
+ * pass of every kind within 20 % of the fastest of all, with and without
+ * programmatic dependent launch (blond_engine_set_overlap), and keeps the
+ * fastest turn (with a beam-phase loop or smooth slicing: the fastest
+ * pass).  Restores the coordinates, the
  * histogram, the turn counter, the induced voltage and the profile.
  * config[9] receives {variant (0 staged, 1 plain, 2 shared table,
  * 3 packed histogram), threads, blocks per SM, histogram
@@ -530,7 +533,8 @@ int blond_batch_check(blond_batch* batch, void* stream);
 int blond_batch_set_shape(blond_batch* batch, int threads, int blocks_per_sm,
                           int particles_per_thread, int chunk, int aggregate);
 /* Time every launch shape above on the bound beams (CUDA events; the
- * coordinates and histograms are restored) and keep the fastest.
+ * fastest few once more, in turn; the coordinates and histograms are
+ * restored) and keep the fastest.
  * config (host, 6 ints) = {threads, blocks_per_sm, particles_per_thread,
  * chunk, aggregate, candidates tried}; best_ms = its particle pass. */
 int blond_batch_autotune(blond_batch* batch, int reps, void* stream, int* config,
