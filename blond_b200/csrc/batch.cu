@@ -207,6 +207,10 @@ particle_kernel_batch(const BatchArgs a) {
         };
         int w = lane_base;
         const int last = 31 + (PP - 1) * bd;  // a full iteration's last pair from w
+        // Worth its instructions' first fetch from eight iterations on (35
+        // beams of 4000 particles, FP64: a turn 24.7 us in the general form
+        // alone, 25.8 with both).
+        const bool plain = !a.agg && npair >= 8 * PP * bd;
         if constexpr (KICK && PP <= 2) {
             // Register pipeline: an iteration's loads are issued while the one
             // before is computed.  With 8 particles a thread the block loads,
@@ -217,7 +221,7 @@ particle_kernel_batch(const BatchArgs a) {
             // 4.9 -> 5.2 TB/s.
             double2 tn[PP];
             E2 en[PP];
-            if (!a.agg && w + last < npair) {
+            if (plain && w + last < npair) {
                 const int j = w + (threadIdx.x & 31);
 #pragma unroll
                 for (int q = 0; q < PP; ++q) {
@@ -253,7 +257,7 @@ particle_kernel_batch(const BatchArgs a) {
                     }
                 }
             }
-        } else if (!a.agg) {
+        } else if (plain) {
             for (; w + last < npair; w += PP * bd) step(w, std::true_type{});
         }
         for (; w < npair; w += PP * bd) step(w, std::false_type{});
@@ -831,9 +835,9 @@ int blond_batch_set_shape(blond_batch* q, int threads, int blocks_per_sm,
 }
 
 // Time every launch shape of the particle pass on the bound beams (CUDA
-// events; one launch each on large batches, else a warm-up and reps; then
-// twice reps launches of the fastest few; the coordinates and histograms
-// restored afterwards) and keep the fastest.  config receives {threads,
+// events; one launch each on large batches, else a warm-up and reps; then the
+// fastest few again, in turn; the coordinates and histograms restored
+// afterwards) and keep the fastest.  config receives {threads,
 // blocks_per_sm, particles_per_thread, chunk, aggregate, candidates}.
 int blond_batch_autotune(blond_batch* q, int reps, void* stream, int* config,
                          double* best_ms) {
@@ -910,7 +914,7 @@ int blond_batch_autotune(blond_batch* q, int reps, void* stream, int* config,
     for (int round = 0; round < 2 && rc == BLOND_OK; ++round)
         for (size_t k = 0; k < order.size() && rc == BLOND_OK; ++k) {
             double ms = 0.0;
-            rc = time_shape(cands[order[k].second], reps, &ms);
+            rc = time_shape(cands[order[k].second], large ? reps : 4 * reps, &ms);
             total[k] += ms / 2;
             if (rc == BLOND_OK && round == 1 && total[k] < best) {
                 best = total[k];
