@@ -85,6 +85,8 @@ particle_kernel_batch(const BatchArgs a) {
     extern __shared__ __align__(16) int sh[];
     TB* stab = reinterpret_cast<TB*>(reinterpret_cast<char*>(sh) + pad16((size_t)a.S * 4));
     __shared__ TurnConsts c;
+    pdl_launch_dependents();
+    pdl_wait();  // the head's table, counter and cleared histograms
     long long t = a.turn ? (*a.turn - 1) : 0;
     if (t < 0) t = 0;
     if (t >= a.n_turns) t = a.n_turns - 1;
@@ -207,10 +209,10 @@ particle_kernel_batch(const BatchArgs a) {
         };
         int w = lane_base;
         const int last = 31 + (PP - 1) * bd;  // a full iteration's last pair from w
-        // Worth its instructions' first fetch from eight iterations on (35
-        // beams of 4000 particles, FP64: a turn 24.7 us in the general form
+        // Worth its instructions' first fetch from four iterations on (35
+        // beams of 4000 particles, FP64: a turn 25.6 us in the general form
         // alone, 25.8 with both).
-        const bool plain = !a.agg && npair >= 8 * PP * bd;
+        const bool plain = !a.agg && npair >= 4 * PP * bd;
         if constexpr (KICK && PP <= 2) {
             // Register pipeline: an iteration's loads are issued while the one
             // before is computed.  With 8 particles a thread the block loads,
@@ -344,6 +346,12 @@ struct blond_batch {
 
 namespace bb {
 
+// Each kernel of a turn launched while the one before it ends (programmatic
+// dependent launch), where the launches show: turns of 4 beams, 8.6e3 particles
+// 11.6 -> 10.2 us, 20 beams, 3.2e6 36.0 -> 34.8, 8 beams, 3.5e6 29.9 -> 28.7; 16
+// beams, 6.4e6 50.6 -> 51.3 (a waiting head holds the SMs' last blocks back).
+static bool batch_overlap(const blond_batch* q) { return q->n_total < (int64_t)1 << 22; }
+
 static BatchArgs batch_args(blond_batch* q) {
     BatchArgs a = {};
     a.dt = q->dt;
@@ -399,7 +407,17 @@ static int launch_batch_k(blond_batch* q, cudaStream_t s, bool launch) {
     if (!launch) return BLOND_OK;
     const int smem = tsm ? tsm : (int)sizeof(int) * q->S;
     const int grid = std::max(1, std::min(q->n_chunks, device_info().sm_count * q->blocks_per_sm));
-    k<<<grid, q->threads, smem, s>>>(batch_args(q));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(q->threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = KICK && batch_overlap(q) ? 1 : 0;
+    BB_CUDA(cudaLaunchKernelEx(&cfg, k, batch_args(q)));
     BB_LAUNCH_CHECK();
     return BLOND_OK;
 }
@@ -499,6 +517,7 @@ static int launch_batch_head(blond_batch* q, cudaStream_t s) {
         C.turn = q->d_turn;
         C.ticket = q->d_cticket;
         C.batch = q->B;
+        C.pdl = batch_overlap(q) ? 1 : 0;
         return launch_conv(C, s);
     }
     SpecParams P = {};
@@ -520,6 +539,7 @@ static int launch_batch_head(blond_batch* q, cudaStream_t s) {
     P.batch = q->B;
     P.beam_scale = q->d_scale;
     P.beam_inv_w = q->d_lik_inv_w;
+    P.pdl = batch_overlap(q) ? 1 : 0;
     return launch_spectral(P, s);
 }
 
