@@ -8,6 +8,10 @@
 #include <stdarg.h>
 #include <math.h>
 
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "../../include/blond_b200.h"
 
 namespace bb {
@@ -66,6 +70,26 @@ struct DeviceInfo {
 };
 // Cached per current device.
 const DeviceInfo& device_info();
+
+// Raise a kernel's dynamic shared memory limit to the opt-in maximum once
+// per (kernel, device).  Never to what one call needs: the limit belongs to
+// the function, so a call of another host thread with a smaller need would
+// lower it between this call's setting and its launch, which then fails.
+template <typename K>
+inline int allow_smem_once(K kernel) {
+    static std::mutex mu;
+    static std::set<std::pair<const void*, int>> done;
+    const DeviceInfo& d = device_info();
+    const std::pair<const void*, int> key(reinterpret_cast<const void*>(kernel), d.device);
+    std::lock_guard<std::mutex> lock(mu);
+    if (done.count(key)) return BLOND_OK;
+    cudaFuncAttributes fa;
+    BB_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    BB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 d.max_smem_optin - (int)fa.sharedSizeBytes));
+    done.insert(key);
+    return BLOND_OK;
+}
 
 // Grid for a grid-stride particle loop: a whole number of waves over the
 // SMs, never more blocks than there are chunks of work.

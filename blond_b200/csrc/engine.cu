@@ -214,24 +214,6 @@ static int launch_tma(blond_engine* e, ParticleArgs a, const TmaPlan& p, cudaStr
     return BLOND_OK;
 }
 
-// Raise a kernel's dynamic shared memory limit to the opt-in maximum once
-// per (kernel, device).
-template <typename K>
-static int allow_smem_once(K kernel) {
-    static std::mutex mu;
-    static std::set<std::pair<const void*, int>> done;
-    const DeviceInfo& d = device_info();
-    const std::pair<const void*, int> key(reinterpret_cast<const void*>(kernel), d.device);
-    std::lock_guard<std::mutex> lock(mu);
-    if (done.count(key)) return BLOND_OK;
-    cudaFuncAttributes fa;
-    BB_CUDA(cudaFuncGetAttributes(&fa, kernel));
-    BB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 d.max_smem_optin - (int)fa.sharedSizeBytes));
-    done.insert(key);
-    return BLOND_OK;
-}
-
 // The plain pass for a histogram mode and prefetch ring depth (0, 2, 4).
 template <int PREC, int SOLVER, bool LIK, bool KICK>
 static auto plain_kernel(bool agg, int ring)

@@ -293,18 +293,19 @@ static int histogram_impl(const T* dt, T* out, T cut_left, T cut_right,
     const size_t smem = sizeof(int) * (size_t)S;
     if ((int64_t)smem <= histogram_smem_budget()) {
         auto launch = [&](auto k, int threads, int per_sm) {
-            const cudaError_t rc = cudaFuncSetAttribute(
-                k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (rc != cudaSuccess) return rc;
+            const int rc = allow_smem_once(k);
+            if (rc) return rc;
             k<<<particle_grid(n, threads, per_sm), threads, smem, s>>>(dt, out, cut_left, inv_w,
                                                                        S, n);
-            return cudaSuccess;
+            return (int)BLOND_OK;
         };
-        BB_CUDA(smem > 32 * 1024
-                    ? (unroll_pays(n) ? launch(histogram_smem_kernel<T, 8, 1024>, 1024, 1)
-                                      : launch(histogram_smem_kernel<T, 1, 1024>, 1024, 1))
-                    : (unroll_pays(n) ? launch(histogram_smem_kernel<T, 8, kThreads>, kThreads, 2)
-                                      : launch(histogram_smem_kernel<T, 1, kThreads>, kThreads, 2)));
+        const int rc =
+            smem > 32 * 1024
+                ? (unroll_pays(n) ? launch(histogram_smem_kernel<T, 8, 1024>, 1024, 1)
+                                  : launch(histogram_smem_kernel<T, 1, 1024>, 1024, 1))
+                : (unroll_pays(n) ? launch(histogram_smem_kernel<T, 8, kThreads>, kThreads, 2)
+                                  : launch(histogram_smem_kernel<T, 1, kThreads>, kThreads, 2));
+        if (rc) return rc;
     } else {
         const int grid = particle_grid(n, 256, 8);
         histogram_global_kernel<T><<<grid, 256, 0, s>>>(dt, out, cut_left, inv_w, S, n);
@@ -362,9 +363,8 @@ static int smooth_histogram_impl(const T* dt, T* out, T cut_left, T cut_right,
     const size_t smem = sizeof(T) * (size_t)S;
     const bool use_smem = (int64_t)smem <= histogram_smem_budget();
     const int grid = particle_grid(n, kThreads, use_smem && smem > 96 * 1024 ? 1 : 2);
-    BB_CUDA(cudaFuncSetAttribute(smooth_histogram_kernel<T>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 use_smem ? (int)smem : 0));
+    const int rc = allow_smem_once(smooth_histogram_kernel<T>);
+    if (rc) return rc;
     smooth_histogram_kernel<T><<<grid, kThreads, use_smem ? smem : 0, s>>>(
         dt, out, cut_left, inv_w, lo, hi, S, n, use_smem);
     BB_LAUNCH_CHECK();
@@ -457,7 +457,8 @@ static int lik_impl(const T* dt, T* dE, const T* V, const T* bc, T charge,
         const bool both = 2 * table <= room;
         auto k = both ? lik_smem_kernel<T, true> : lik_smem_kernel<T, false>;
         const int smem = (int)(both ? 2 * table : table);
-        BB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        const int rc = allow_smem_once(k);
+        if (rc) return rc;
         k<<<particle_grid(n, kLikThreads, 1), kLikThreads, smem, s>>>(dt, dE, V, bc, charge, S, n,
                                                                       acc);
     } else {
