@@ -67,7 +67,9 @@ class RingAndRFTracker:
     def kick(self, beam_dt, beam_dE, index: int):
         """tracker.py:399-422."""
         V, om, ph = self._programme()
-        if beam_dt.dtype != V.dtype or not 0 <= index < V.shape[0]:
+        # another type or GPU than the programme's copy: its row is converted
+        if beam_dt.dtype != V.dtype or beam_dt.device != V.device \
+                or not 0 <= index < V.shape[0]:
             return bm.kick(beam_dt, beam_dE, V[index], om[index], ph[index],
                            self.rf_params.particle.charge, self.rf_params.n_rf,
                            self.acceleration_kick[index])
