@@ -105,14 +105,21 @@ class RingAndRFTracker:
         if self.beamFB is not None and turn >= self.beamFB.delay:
             self.beamFB.track()
             self._sync_column(1, turn + 1)
-        # (element by element: numpy's calls on arrays of n_rf took 8 us a turn)
-        shifted = False
-        for j in range(rf.n_rf):
-            design = rf.omega_rf_d[j, turn + 1]
-            dphi = rf.dphi_rf[j] + (2.0 * np.pi * rf.harmonic[j, turn + 1]
-                                    * (rf.omega_rf[j, turn + 1] - design) / design)
-            rf.dphi_rf[j] = dphi
-            shifted = shifted or dphi != 0
+        if isinstance(rf.dphi_rf, np.ndarray) and rf.dphi_rf.dtype == np.float64 \
+                and rf.dphi_rf.shape == (rf.n_rf,):
+            # (element by element: numpy's calls on arrays of n_rf took 8 us a turn)
+            shifted = False
+            for j in range(rf.n_rf):
+                design = rf.omega_rf_d[j, turn + 1]
+                dphi = rf.dphi_rf[j] + (2.0 * np.pi * rf.harmonic[j, turn + 1]
+                                        * (rf.omega_rf[j, turn + 1] - design) / design)
+                rf.dphi_rf[j] = dphi
+                shifted = shifted or dphi != 0
+        else:  # a number, or another type of array, put there by the program
+            rf.dphi_rf += (2.0 * np.pi * rf.harmonic[:, turn + 1]
+                           * (rf.omega_rf[:, turn + 1] - rf.omega_rf_d[:, turn + 1])
+                           / rf.omega_rf_d[:, turn + 1])
+            shifted = np.any(rf.dphi_rf != 0)
         if shifted:
             rf.phi_rf[:, turn + 1] += rf.dphi_rf
             self._sync_phase(turn + 1)

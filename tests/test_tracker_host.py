@@ -44,3 +44,40 @@ def test_kick_passes_addresses_only_to_arrays_beside_them(monkeypatch, device, d
     else:
         assert kind == "row"
         assert all(torch.equal(x, y[index]) for x, y in zip(a[2:5], (V, om, ph)))
+
+
+def _phase_after_a_turn(dphi_rf, offset, monkeypatch):
+    """phi_rf of the next turn and dphi_rf after one turn that starts with
+    ``dphi_rf`` and has the frequency ``offset`` beside the design one."""
+    rf, tracker = _tracker()
+    rf.empty = True  # no kick
+    monkeypatch.setattr(bm, "drift", lambda *a: None)
+    rf.omega_rf[:, 1] += np.asarray(offset)
+    rf.dphi_rf = dphi_rf
+    tracker.track()
+    return rf.phi_rf[:, 1], rf.dphi_rf
+
+
+@pytest.mark.parametrize("dphi", [np.zeros(2), np.array([0.25, -0.5]), 0.25, np.float64(0.5),
+                                  np.array([0.5, 0.25], np.float32),
+                                  np.array([0.5, np.nan])],
+                         ids=["zeros", "values", "float", "scalar", "float32", "nan"])
+@pytest.mark.parametrize("offset", [[0.0, 0.0], [1e3, -2e3]], ids=["design", "offset"])
+def test_phase_offset_of_every_kind(monkeypatch, dphi, offset):
+    """The frequency offset's phase is added to dphi_rf, as an array expression
+    over the RF systems adds it, and the sum to the next turn's phase."""
+    rf, _ = _tracker()
+    od, h = rf.omega_rf_d[:, 1], rf.harmonic[:, 1]
+    om = rf.omega_rf[:, 1] + np.asarray(offset)
+    want = dphi.copy() if isinstance(dphi, np.ndarray) else dphi
+    want += 2.0 * np.pi * h * (om - od) / od
+    phi, got = _phase_after_a_turn(dphi, offset, monkeypatch)
+    np.testing.assert_array_equal(got, want)
+    assert np.asarray(got).dtype == np.asarray(want).dtype
+    np.testing.assert_array_equal(phi, rf.phi_rf[:, 1] + want)
+
+
+def test_phase_offset_of_whole_numbers_is_refused(monkeypatch):
+    """Fractions of a radian cannot be added to an integer array in place."""
+    with pytest.raises(TypeError):
+        _phase_after_a_turn(np.zeros(2, int), [1e3, 0.0], monkeypatch)
