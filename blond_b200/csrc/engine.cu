@@ -982,7 +982,9 @@ static int launch_multi_p(blond_engine* e, const ParticleArgs& a, int first, int
 
 // n_turns turns in launches of at most kMultiTurns, evenly split; the
 // histogram, profile and turn counter end as after n_turns single turns.
+// Options that a single turn's pass refuses are refused here too.
 static int run_multi(blond_engine* e, int64_t n_turns, cudaStream_t s) {
+    if (const int refused = launch_particles(e, true, s, false)) return refused;
     ParticleArgs a = particle_args(e);
     // the constants of a launch's turns lie before the block's histogram
     a.global_hist = (size_t)e->S * sizeof(int) + sizeof(TurnConsts) * kMultiTurns + 1024 >
@@ -1795,7 +1797,9 @@ int blond_engine_prepare(blond_engine* e, void* stream) {
     BB_CHECK_ARG(e, "engine_prepare: null engine");
     int rc = check_ready(e);
     if (rc) return rc;
-    if (e->turns_per_graph <= 1 || multi_turn(e)) return BLOND_OK;
+    if (e->turns_per_graph <= 1) return BLOND_OK;
+    // no graph, but what tracking would refuse is refused here
+    if (multi_turn(e)) return launch_particles(e, true, as_stream(stream), false);
     return ensure_graph(e, as_stream(stream));
 }
 
