@@ -282,14 +282,18 @@ bool make_conv_plan(int S, int64_t N, int B, ConvPlan& plan) {
 }
 
 // hx[b][x] = y[b][(x - (S - 1)) mod N]
-__global__ void conv_response_kernel(const double* y, int64_t N, int S, double* hx) {
-    const int64_t b = blockIdx.y;
-    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < 2 * S - 1;
-         x += (int64_t)gridDim.x * blockDim.x) {
-        int64_t d = x - (S - 1);
-        if (d < 0) d += N;
-        hx[b * (2 * S - 1) + x] = y[b * N + d];
-    }
+__global__ void conv_response_kernel(const double* y, int64_t N, int S, int B, double* hx) {
+    for (int64_t b = blockIdx.y; b < B; b += gridDim.y)
+        for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < 2 * S - 1;
+             x += (int64_t)gridDim.x * blockDim.x) {
+            int64_t d = x - (S - 1);
+            if (d < 0) d += N;
+            hx[b * (2 * S - 1) + x] = y[b * N + d];
+        }
+}
+// A grid has at most 65535 rows: more beams than that share them.
+static dim3 response_grid(int S, int B) {
+    return dim3((2 * S + 254) / 256, std::min(B, 65535));
 }
 
 int make_conv_response(const double2* H, int64_t N, int S, int B, double** hx) {
@@ -306,7 +310,7 @@ int make_conv_response(const double2* H, int64_t N, int S, int B, double** hx) {
         rc = BLOND_ERR_CUDA;
     }
     if (rc == BLOND_OK) {
-        conv_response_kernel<<<dim3((2 * S + 254) / 256, B), 256>>>(y, N, S, *hx);
+        conv_response_kernel<<<response_grid(S, B), 256>>>(y, N, S, B, *hx);
         if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
             set_error("convolution head: response kernel failed");
             rc = BLOND_ERR_CUDA;
@@ -324,7 +328,7 @@ int conv_response_async(const double2* H, int64_t N, int S, double* y, double* h
                         cudaStream_t stream) {
     const int rc = blond_irfft_f64(reinterpret_cast<const double*>(H), N, y, N, stream);
     if (rc) return rc;
-    conv_response_kernel<<<dim3((2 * S + 254) / 256, 1), 256, 0, stream>>>(y, N, S, hx);
+    conv_response_kernel<<<response_grid(S, 1), 256, 0, stream>>>(y, N, S, 1, hx);
     BB_LAUNCH_CHECK();
     return BLOND_OK;
 }
