@@ -83,18 +83,22 @@ conv_head_kernel(const ConvParams P, const typename ConvLoopArg<FB>::type fb) {
             }
         }
     }
+    // with the loop the extra warp leaves the profile to the others: reading it
+    // too, after its sums, held the block barrier back (0.5 us of a turn at 200
+    // to 9000 slices)
     const int nfill = FB ? nth : nth + 32;
+    const int end = tid < nfill ? T : 0;
     if (P.in_i32) {
         const int* const in = P.in_i32 + boff;
-        fill_shared(prof, T, tid, nfill, [&](int j) { return j < S ? __ldcg(in + j) : 0; });
+        fill_shared(prof, end, tid, nfill, [&](int j) { return j < S ? __ldcg(in + j) : 0; });
     } else if (P.in_fix) {
         const unsigned long long* const in = P.in_fix + boff;
-        fill_shared(prof, T, tid, nfill, [&](int j) {
+        fill_shared(prof, end, tid, nfill, [&](int j) {
             return j < S ? (double)__ldcg(in + j) * P.fix_unit : 0.0;
         });
     } else {
         const double* const in = P.in_f64 + boff;
-        fill_shared(prof, T, tid, nfill, [&](int j) { return j < S ? __ldcg(in + j) : 0.0; });
+        fill_shared(prof, end, tid, nfill, [&](int j) { return j < S ? __ldcg(in + j) : 0.0; });
     }
     __syncthreads();
     if (tid >= nth) {
