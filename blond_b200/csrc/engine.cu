@@ -230,6 +230,11 @@ static auto plain_kernel(bool agg, int ring)
                : particle_kernel<PREC, SOLVER, LIK, KICK, false, 0>;
 }
 
+// The packed pass's prefetch setting that means the register pipeline; the
+// other passes take it as direct loads.
+constexpr int kPipeRing = 1;
+static int ring_stages(const blond_engine* e) { return e->ring == kPipeRing ? 0 : e->ring; }
+
 // Dynamic shared memory of the plain pass: the histogram (16-byte aligned)
 // and the prefetch ring; -1 if that exceeds the opt-in limit.
 template <int PREC>
@@ -271,15 +276,12 @@ static auto packed_kernel() {
     return particle_kernel_stab<PREC, SOLVER, NST, TAB>;
 }
 
-// The packed pass's prefetch setting that means the register pipeline.
-constexpr int kPipeRing = 1;
-
 template <int PREC, int SOLVER>
 static int launch_stab(blond_engine* e, const ParticleArgs& a, cudaStream_t s, bool launch) {
     const bool shared = e->variant == 2;
     const bool pipe = !shared && e->ring == kPipeRing;
-    const int ring = shared ? (e->ring ? 2 : 0)
-                            : (e->ring >= 4 ? 4 : (e->ring && !pipe ? 2 : 0));
+    const int stages = ring_stages(e);
+    const int ring = shared ? (stages ? 2 : 0) : (stages >= 4 ? 4 : (stages ? 2 : 0));
     const int smem = shared ? stab_smem<PREC>(e, ring) : packed_smem<PREC>(e, ring);
     if (smem < 0) {
         set_error(shared ? "engine: the shared-table pass does not apply to this engine"
@@ -354,7 +356,7 @@ static int launch_particles_t(blond_engine* e, const ParticleArgs& a, cudaStream
     int grid = particle_grid(a.n / 2 + 1, e->threads, e->blocks_per_sm);
     const int cl = plain_global(e) ? 1 : e->cluster;  // merging needs shared histograms
     grid = (grid + cl - 1) / cl * cl;
-    const int ring = KICK ? e->ring : 0;
+    const int ring = KICK ? ring_stages(e) : 0;
     auto k = plain_kernel<PREC, SOLVER, LIK, KICK>(agg, ring);
     if ((rc = allow_smem_once(k))) return rc;
     const int smem_ring = plain_ring_smem<PREC>(e, ring);
@@ -670,8 +672,9 @@ particle_kernel_smooth(const ParticleArgs a, double lo, double hi, double scale,
 // then follow each other.
 static int smooth_pass_smem(const blond_engine* e) {
     if (!e->smooth || e->variant == 2 || e->variant == 3) return -1;
-    if (e->ring && (e->precision == BLOND_PREC_F64 ? plain_ring_smem<PREC_F64>(e, e->ring)
-                                                   : plain_ring_smem<PREC_F32P64>(e, e->ring)) < 0)
+    const int ring = ring_stages(e);
+    if (ring && (e->precision == BLOND_PREC_F64 ? plain_ring_smem<PREC_F64>(e, ring)
+                                                : plain_ring_smem<PREC_F32P64>(e, ring)) < 0)
         return -1;
     const size_t bytes = 8 * (size_t)e->S;
     const size_t limit = (size_t)device_info().max_smem_optin - sizeof(TurnConsts) - 1024;
@@ -1453,8 +1456,9 @@ int blond_engine_set_overlap(blond_engine* e, int on) {
 }
 
 int blond_engine_set_prefetch(blond_engine* e, int stages) {
-    BB_CHECK_ARG(e && (stages == 0 || stages == 2 || stages == 4),
-                 "engine_set_prefetch: stages must be 0, 2 or 4");
+    BB_CHECK_ARG(e && (stages == 0 || stages == kPipeRing || stages == 2 || stages == 4),
+                 "engine_set_prefetch: stages must be 0, 2 or 4 (or 1, what the autotuner "
+                 "calls the packed pass's register pipeline)");
     e->ring = stages;
     e->graph_dirty = true;
     return BLOND_OK;

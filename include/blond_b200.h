@@ -453,8 +453,10 @@ int blond_engine_tune(blond_engine* engine, int threads, int blocks_per_sm,
  * packed 16-bit counters (staged pass), 3 global-memory atomics (plain
  * pass).  A layout that does not fit falls back to the automatic one. */
 int blond_engine_set_histogram(blond_engine* engine, int mode);
-/* Plain pass: depth of the per-thread cp.async prefetch ring (0 = direct
- * loads, 2 or 4 stages). */
+/* Plain, shared-table and packed pass: depth of the per-thread cp.async
+ * prefetch ring (0 = direct loads, 2 or 4 stages).  1, as the autotuner
+ * reports it, is the packed pass's register pipeline and direct loads in the
+ * others. */
 int blond_engine_set_prefetch(blond_engine* engine, int stages);
 /* Shared-table pass: thread 0 of each block also prefetches the block's
  * slice one iteration beyond the ring into L2 (cp.async.bulk.prefetch);
