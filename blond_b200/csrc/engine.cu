@@ -1231,7 +1231,18 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
                   (long long)n_fft);
     BB_CHECK_SIZE(n_fft >= e->S, "engine_set_impedance: n_fft=%lld shorter than the "
                   "profile (%d slices)", (long long)n_fft, e->S);
-    int rc = upload((void**)&e->d_H, Z, sizeof(double2) * (size_t)(n_fft / 2 + 1));
+    // Everything is built beside what the engine has and put in its place at
+    // the end: a call that fails changes nothing.
+    struct Built {
+        double2 *H = nullptr, *tw = nullptr;
+        double* hx = nullptr;
+        ~Built() {
+            free_ptr(H);
+            free_ptr(tw);
+            free_ptr(hx);
+        }
+    } b;
+    int rc = upload((void**)&b.H, Z, sizeof(double2) * (size_t)(n_fft / 2 + 1));
     if (rc) return rc;
     // Short profiles: the direct convolution's impulse response.  Not in
     // Q32P64: where its voltages round otherwise in the last bit, a few
@@ -1239,31 +1250,35 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
     // repeat one of an earlier build.  Its head stays the cluster FFT with
     // that kernel's roundings (2e4 particles, 2000 slices 24 us a turn, 9 with
     // the convolution; 1e8 particles, 2^16 slices: 1 % of the turn).
-    e->conv = false;
-    free_ptr(e->d_hx);
-    e->d_hx = nullptr;
-    if (e->precision != BLOND_PREC_Q32P64 && make_conv_plan(e->S, n_fft, 1, e->cplan)) {
+    ConvPlan cplan;
+    const bool conv =
+        e->precision != BLOND_PREC_Q32P64 && make_conv_plan(e->S, n_fft, 1, cplan);
+    if (conv) {
         if (!e->d_cticket) {
-            BB_CUDA(cudaMalloc((void**)&e->d_cticket, sizeof(int)));
+            int* ticket = nullptr;
+            BB_CUDA(cudaMalloc((void**)&ticket, sizeof(int)));
+            e->d_cticket = ticket;
             BB_CUDA(cudaMemset(e->d_cticket, 0, sizeof(int)));
         }
-        if ((rc = make_conv_response(e->d_H, n_fft, e->S, 1, &e->d_hx))) return rc;
+        if ((rc = make_conv_response(b.H, n_fft, e->S, 1, &b.hx))) return rc;
         if ((rc = prepare_conv())) return rc;
-        e->conv = true;
     } else if (const int64_t P =
                    e->precision != BLOND_PREC_Q32P64 ? head_fft_length(n_fft, e->S) : 0) {
         // long profiles at other lengths: the same voltages by the
         // power-of-two transform
         double2* H = nullptr;
-        if ((rc = make_head_response(e->d_H, n_fft, e->S, P, &H))) return rc;
-        free_ptr(e->d_H);
-        e->d_H = H;
+        if ((rc = make_head_response(b.H, n_fft, e->S, P, &H))) return rc;
+        free_ptr(b.H);
+        b.H = H;
         make_spec_plan(P, plan);
     }
     // twiddle tables of this plan, computed once instead of every turn
-    free_ptr(e->d_tw);
-    e->d_tw = nullptr;
-    if ((rc = make_spec_twiddles(plan, &e->d_tw))) return rc;
+    if ((rc = make_spec_twiddles(plan, &b.tw))) return rc;
+    std::swap(e->d_H, b.H);
+    std::swap(e->d_tw, b.tw);
+    std::swap(e->d_hx, b.hx);
+    e->conv = conv;
+    e->cplan = cplan;
     e->plan = plan;
     e->iv_scale = scale;
     e->has_fft = true;
