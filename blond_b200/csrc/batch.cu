@@ -743,33 +743,49 @@ int blond_batch_set_impedance(blond_batch* q, int64_t n_fft, const double* Z,
     BB_CHECK_SIZE(n_fft >= q->S && plan.smem <= device_info().max_smem_optin,
                   "batch_set_impedance: n_fft=%lld unsupported for %d slices",
                   (long long)n_fft, q->S);
+    // built beside what the batch has and put in its place at the end, as in
+    // blond_engine_set_impedance
+    struct Built {
+        double2 *H = nullptr, *tw = nullptr;
+        double *scale = nullptr, *cscale = nullptr, *hx = nullptr;
+        ~Built() {
+            for (void* p : {(void*)H, (void*)tw, (void*)scale, (void*)cscale, (void*)hx})
+                free_ptr(p);
+        }
+    } n;
     std::vector<double> sc(q->B);
     for (int b = 0; b < q->B; ++b) sc[b] = -scale[b] / (double)plan.M;
     int rc;
-    if ((rc = upload((void**)&q->d_H, Z, sizeof(double2) * (size_t)q->B * (n_fft / 2 + 1))))
+    if ((rc = upload((void**)&n.H, Z, sizeof(double2) * (size_t)q->B * (n_fft / 2 + 1))))
         return rc;
-    if ((rc = upload((void**)&q->d_scale, sc.data(), sizeof(double) * q->B))) return rc;
-    free_ptr(q->d_tw);
-    q->d_tw = nullptr;
-    if ((rc = make_spec_twiddles(plan, &q->d_tw))) return rc;
-    q->plan = plan;
-    q->has_fft = true;
+    if ((rc = upload((void**)&n.scale, sc.data(), sizeof(double) * q->B))) return rc;
+    if ((rc = make_spec_twiddles(plan, &n.tw))) return rc;
     // short profiles: the direct convolution's impulse responses (not in
     // Q32P64, as in blond_engine_set_impedance)
-    q->conv = false;
-    free_ptr(q->d_hx);
-    q->d_hx = nullptr;
-    if (q->precision != BLOND_PREC_Q32P64 && make_conv_plan(q->S, n_fft, q->B, q->cplan)) {
+    ConvPlan cplan;
+    const bool conv =
+        q->precision != BLOND_PREC_Q32P64 && make_conv_plan(q->S, n_fft, q->B, cplan);
+    if (conv) {
         for (int b = 0; b < q->B; ++b) sc[b] = -scale[b];
-        if ((rc = upload((void**)&q->d_cscale, sc.data(), sizeof(double) * q->B))) return rc;
+        if ((rc = upload((void**)&n.cscale, sc.data(), sizeof(double) * q->B))) return rc;
         if (!q->d_cticket) {
-            BB_CUDA(cudaMalloc((void**)&q->d_cticket, sizeof(int) * q->B));
+            int* ticket = nullptr;
+            BB_CUDA(cudaMalloc((void**)&ticket, sizeof(int) * q->B));
+            q->d_cticket = ticket;
             BB_CUDA(cudaMemset(q->d_cticket, 0, sizeof(int) * q->B));
         }
-        if ((rc = make_conv_response(q->d_H, n_fft, q->S, q->B, &q->d_hx))) return rc;
+        if ((rc = make_conv_response(n.H, n_fft, q->S, q->B, &n.hx))) return rc;
         if ((rc = prepare_conv())) return rc;
-        q->conv = true;
     }
+    std::swap(q->d_H, n.H);
+    std::swap(q->d_tw, n.tw);
+    std::swap(q->d_scale, n.scale);
+    std::swap(q->d_cscale, n.cscale);
+    std::swap(q->d_hx, n.hx);
+    q->conv = conv;
+    q->cplan = cplan;
+    q->plan = plan;
+    q->has_fft = true;
     q->graph_dirty = true;
     return BLOND_OK;
 }
