@@ -7,8 +7,12 @@ scan over hundreds of such beams (different voltages, bunch lengths,
 impedances; ragged particle counts) then costs hundreds of small launches
 per turn.  ``BatchTracker`` takes the drop-in objects of all beams and
 tracks them with the batched engine (blond_batch_*): one particle pass and
-one head launch (one FFT cluster per beam) per turn, replayed from a CUDA
-graph, each beam with the single-beam engine's arithmetic.
+one head launch (one FFT cluster per beam, or its direct convolution) per turn,
+replayed from a CUDA graph, each beam with the single-beam engine's particle
+arithmetic.  F64 and F32P64 beams have the single-beam engine's bits as long as
+both convolve: profiles of up to 4600 slices in batches of up to 8, or with
+n_beams * n_slices**2 up to 8e6.  Beyond, the two may transform in different
+kernels, and the induced voltages agree within rounding.
 
 All beams must share the number of RF systems, the drift solver, the
 number of slices, the programme length and (when present) the FFT length

@@ -262,8 +262,12 @@ bool make_conv_plan(int S, int64_t N, int B, ConvPlan& plan) {
     if (B == 1 && pow2 && S > 4600) return false;
     // a batch: the profiles' multiply-adds share the SMs (37 beams of 400
     // slices 21.2 -> 14.5 us a turn, but 64 of 512 would be 16 -> 23 and 256 of
-    // 300 37 -> 40); up to 8 beams take the single beam's rule, so that they
-    // also take its bits
+    // 300 37 -> 40); up to 8 beams of up to 4600 slices convolve as single ones
+    // do.  A beam of a batch has the single-beam engine's bits where both
+    // convolve; elsewhere the batch takes spectral_kernel and the single beam
+    // may take another head (9000 slices: convolution; 8192 and 14000: the
+    // 16-CTA transform; 512 in a batch of 64: convolution), and the voltages
+    // agree within the two heads' rounding, 4e-14 of the largest.
     if (B > 1 && (int64_t)B * S * S > 8'000'000 && (B > 8 || S > 4600)) return false;
     int g = 1;
     while (g < kConvMaxGroups && (kConvTile * g - 1) * sms < S) ++g;
