@@ -38,10 +38,13 @@ def _objects(n, S, seed):
 
 
 # single / batch: convolution / mixed radix (9000, 12000), padded transform /
-# mixed radix (14000), convolution / power of two (64 of 512), convolution both
-# with other tiles per block (150 of 64)
-@pytest.mark.parametrize("B,S", [(2, 9000), (3, 12000), (2, 14000), (64, 512), (150, 64)])
-def test_same_voltages_as_single_beams(cuda, B, S):
+# mixed radix (14000), 16-CTA / general transform (8192), convolution / power of
+# two (64 of 512); convolution both, with other tiles per block (150 of 64, 37 of
+# 400, 8 of 4096): equal bits
+@pytest.mark.parametrize("B,S,same", [(2, 9000, False), (3, 12000, False), (2, 14000, False),
+                                      (3, 8192, False), (64, 512, False), (150, 64, True),
+                                      (37, 400, True), (8, 4096, True)])
+def test_same_voltages_as_single_beams(cuda, B, S, same):
     batch = BatchTracker([_objects(3000 + b, S, b) for b in range(B)], precision="f64")
     singles = [FusedTracker(*_objects(3000 + b, S, b), precision="f64")
                for b in range(0, B, max(1, B // 5))]
@@ -53,6 +56,9 @@ def test_same_voltages_as_single_beams(cuda, B, S):
         top = float(v.abs().max())
         assert top > 0
         assert float((V[b] - v).abs().max()) <= 4e-14 * top
+        if same:
+            assert torch.equal(V[b], v)
+            assert torch.equal(batch.coordinates(b)[1], one.dE)
         assert torch.equal(p[b], one.profile_tensor())
         dE = batch.coordinates(b)[1]
         eps = np.finfo(float).eps
