@@ -1265,7 +1265,12 @@ int blond_engine_set_impedance(blond_engine* e, int64_t n_fft, const double* Z,
     } else if (const int64_t P =
                    e->precision != BLOND_PREC_Q32P64 ? head_fft_length(n_fft, e->S) : 0) {
         // long profiles at other lengths: the same voltages by the
-        // power-of-two transform
+        // power-of-two transform.  Also with a beam-phase loop, whose head is
+        // spectral_kernel with either length: its warp transforms of powers of
+        // two outweigh the longer one (turns of 1e5 FP64 particles with the
+        // loop, n_fft itself -> P: 14000 slices 66.2 -> 34.5 us, 16000 47.1 ->
+        // 36.2, 20000 81.2 -> 51.0, 40000 138.3 -> 87.7; without it 54.0 ->
+        // 23.7, 37.8 -> 24.8, 68.4 -> 34.3, 113.6 -> 62.5)
         double2* H = nullptr;
         if ((rc = make_head_response(b.H, n_fft, e->S, P, &H))) return rc;
         free_ptr(b.H);
@@ -1736,9 +1741,10 @@ int blond_engine_autotune(blond_engine* e, int reps, void* stream, int* config,
         }
     // whole turns: every kind of pass within 20 % of the fastest, overlap on
     // or off -- what a pass asks of the head and how much of it the pass
-    // overlaps count as well (Q32P64, 1e7 particles, 16384 slices: the packed
-    // pass is the faster one alone, but its turn takes 70 us, the shared-table
-    // pass's 65)
+    // overlaps count as well (Q32P64, 1e7 particles, 16384 slices, turns: the
+    // packed pass's register pipeline 68.0 us, the shared-table pass, whose head
+    // writes no table, 70.0, the packed pass without it 70.8 to 73.8, the plain
+    // pass 74.9)
     auto apply = [&](const Cand& c) {
         e->variant = c.variant;
         e->threads = c.threads;

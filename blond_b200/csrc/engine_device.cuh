@@ -745,7 +745,8 @@ particle_kernel(const ParticleArgs a) {
 // Each turn runs track_pair with its own constants, the same operations as
 // one pass per turn.  Bound: FP64 issue (24 float64 operations per particle
 // and turn at one RF system: 133 us for 100 turns of 1e6 particles; measured
-// 180 us, 873 us with two launches per turn).  The turn counter is read, not
+// 165 us, 850 us with two launches per turn; ncu: FP64 pipe 73 % busy, its
+// throttle the top stall).  The turn counter is read, not
 // advanced: `first` is this launch's offset from it.
 // NRF: 1 or 2 RF systems written out, 0 the run-time count.
 constexpr int kMultiTurns = 64;  // turns per launch, at most
@@ -1007,8 +1008,11 @@ particle_kernel_stab(const ParticleArgs a) {
 // computes one pair, the table entries of its next pair and the coordinates of
 // the one after are on their way.  Long profiles gather from L2 (1 MB at 2^16
 // slices) and leave no shared memory for a ring, so the pass above waits for
-// both one after the other (ncu: 4.5 long-scoreboard stalls per issue, issue
-// active 61 %).  768 threads: 80 registers.
+// both one after the other (ncu: 3.6 long-scoreboard stalls per issue, 0.5
+// here).  768 threads: 80 registers.  Bound: no one unit.  2e7 Q32P64 particles,
+// 2^16 slices, double RF: requests from L1 to L2 69 % of their peak, issue 62 %,
+// FP64 40 %, DRAM 34 %; the stalls are `wait` (2.9) and the shared deposits'
+// short scoreboard (2.4) at 24 warps an SM.
 constexpr int kPipeThreads = 768;
 
 template <int PREC, int SOLVER>
