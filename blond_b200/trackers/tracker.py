@@ -19,6 +19,9 @@ import torch
 
 from .. import bmath as bm
 
+_TWO_PI = 2.0 * np.pi
+_F64 = np.dtype(np.float64)
+
 
 class RingAndRFTracker:
     def __init__(self, rf_station, beam, solver: str = "simple",
@@ -105,15 +108,15 @@ class RingAndRFTracker:
         if self.beamFB is not None and turn >= self.beamFB.delay:
             self.beamFB.track()
             self._sync_column(1, turn + 1)
-        if isinstance(rf.dphi_rf, np.ndarray) and rf.dphi_rf.dtype == np.float64 \
-                and rf.dphi_rf.shape == (rf.n_rf,):
+        offset = rf.dphi_rf
+        if type(offset) is np.ndarray and offset.dtype is _F64 and offset.shape == (rf.n_rf,):
             # (element by element: numpy's calls on arrays of n_rf took 8 us a turn)
             shifted = False
+            nxt, omega, design, harmonic = turn + 1, rf.omega_rf, rf.omega_rf_d, rf.harmonic
             for j in range(rf.n_rf):
-                design = rf.omega_rf_d[j, turn + 1]
-                dphi = rf.dphi_rf[j] + (2.0 * np.pi * rf.harmonic[j, turn + 1]
-                                        * (rf.omega_rf[j, turn + 1] - design) / design)
-                rf.dphi_rf[j] = dphi
+                d = design[j, nxt]
+                dphi = offset[j] + _TWO_PI * harmonic[j, nxt] * (omega[j, nxt] - d) / d
+                offset[j] = dphi
                 shifted = shifted or dphi != 0
         else:  # a number, or another type of array, put there by the program
             rf.dphi_rf += (2.0 * np.pi * rf.harmonic[:, turn + 1]
